@@ -338,7 +338,7 @@ void LaunchCore::release() {
                         &d_post_views, &d_draws, &d_scenes, &clip, &world, &normal, &color,
                         &rrec, &srec, &clipq, &large_list, &large_items, &keys, &shade_list,
                         &pre, &out, &depth, &ids, &presented, &hdr, &frag_head, &touched,
-                        &frags, &olist, &olist_items, &wlist, &wlist_items, &oscratch};
+                        &frags, &olist, &olist_items, &wlist, &wlist_items, &wplots, &oscratch};
   for (DevArena *a : arenas)
     a->release();
   frag_pool = olist_pool = wlist_pool = 0;
@@ -370,7 +370,7 @@ void LaunchCore::trim() {
                         &clipq,      &large_list, &large_items, &keys, &shade_list, &pre,
                         &out,        &depth, &ids,     &presented,  &hdr,       &frag_head,
                         &touched,    &frags, &olist,   &olist_items, &wlist, &wlist_items,
-                        &oscratch};
+                        &wplots,     &oscratch};
   for (DevArena *a : arenas)
     a->release();
   vertex_pool = rec_pool = clip_pool = large_pool = 0;
@@ -383,7 +383,7 @@ uint64_t LaunchCore::device_bytes() const {
                               &rrec, &srec, &clipq, &large_list, &large_items, &keys,
                               &shade_list, &pre, &out, &depth, &ids, &presented, &hdr,
                               &frag_head, &touched, &frags, &olist, &olist_items, &wlist,
-                              &wlist_items, &oscratch};
+                              &wlist_items, &wplots, &oscratch};
   uint64_t t = 0;
   for (const DevArena *a : arenas)
     t += a->cap;
@@ -678,8 +678,8 @@ int LaunchCore::stage_suffix() {
     }
   }
   const unsigned long long sa = std::max(total_samples, sample_floor);
-  void *before[9] = {hdr.p, frag_head.p, touched.p, frags.p, olist.p, olist_items.p,
-                     wlist.p, wlist_items.p, oscratch.p};
+  void *before[10] = {hdr.p, frag_head.p, touched.p, frags.p, olist.p, olist_items.p,
+                      wlist.p, wlist_items.p, wplots.p, oscratch.p};
   int rc = 0;
   rc |= hdr.ensure(16ull * sa);
   rc |= frag_head.ensure(4ull * sa);
@@ -701,8 +701,10 @@ int LaunchCore::stage_suffix() {
   olist_pool = std::min(olist.cap / 4, olist_items.cap / 4);
   frag_pool = std::min(frags.cap / 8, oscratch.cap / 16);
   wlist_pool = std::min(wlist.cap / 4, wlist_items.cap / 4);
-  void *after_[9] = {hdr.p, frag_head.p, touched.p, frags.p, olist.p, olist_items.p,
-                     wlist.p, wlist_items.p, oscratch.p};
+  if (any_wire && wplots.ensure(sizeof(WirePlot) * frag_pool))
+    return MOPCUDA_ENOMEM;
+  void *after_[10] = {hdr.p, frag_head.p, touched.p, frags.p, olist.p, olist_items.p,
+                      wlist.p, wlist_items.p, wplots.p, oscratch.p};
   if (memcmp(before, after_, sizeof before) != 0)
     suffix_moved = true;
   return MOPCUDA_OK;
@@ -769,6 +771,7 @@ int LaunchCore::enqueue(int parts) {
       a.wlist = wlist.as<uint32_t>();
       a.wlist_items = wlist_items.as<uint32_t>();
       a.wlist_pool = wlist_pool;
+      a.wplots = wplots.as<WirePlot>();
     }
   }
 
@@ -905,6 +908,8 @@ int LaunchCore::after(bool *rerun, int attempt) {
       rc |= oscratch.ensure(16ull * fr);
       frag_pool = std::min(frags.cap / 8, oscratch.cap / 16);
     }
+    if (any_wire)
+      rc |= wplots.ensure(sizeof(WirePlot) * frag_pool);
     if (rc)
       return MOPCUDA_ENOMEM;
   }

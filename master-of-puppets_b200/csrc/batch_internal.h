@@ -83,7 +83,8 @@ struct LaunchCore {
    * launch its per-sample buffers and pools; suffix_moved: stage()
    * reallocated one of them */
   bool any_ordered = false, any_wire = false, suffix_moved = false;
-  DevArena hdr, frag_head, touched, frags, olist, olist_items, wlist, wlist_items, oscratch;
+  DevArena hdr, frag_head, touched, frags, olist, olist_items, wlist, wlist_items, wplots,
+      oscratch;
   unsigned long long frag_pool = 0, olist_pool = 0, wlist_pool = 0;
   uint32_t frag_num = 4;
   uint32_t post_count[4] = {0, 0, 0, 0}, post_tiles[4] = {0, 0, 0, 0};

@@ -1978,6 +1978,8 @@ template <bool SH, bool WIRE> __global__ void k_ofold(FrameArgs a);
 __global__ void k_wcount(FrameArgs a);
 __global__ void k_wscan(FrameArgs a);
 __global__ void k_wplot(FrameArgs a);
+#define WLONG_WARPS 4 /* warps of a k_wlong block */
+template <bool SH> __global__ void k_wlong(FrameArgs a);
 
 /* The legacy smooth path's shading (mop_sw_rasterize_triangle_smooth,
  * rasterizer.c:1371-1420): interpolated normal and vertex colour, one
@@ -2072,10 +2074,14 @@ int mopcuda_launch_frame(const FrameArgs &a, const PostArgs &p, const LaunchCfg 
       pdl(k_wscan, 1, 1024, s, a);
       pdl(k_wplot, cfg.num_sms * 8, 256, s, a);
       launches += 3;
-      if (a.shadow_keys)
+      if (a.shadow_keys) {
         pdl(k_ofold<true, true>, cfg.num_sms * 8, 128, s, a);
-      else
+        pdl(k_wlong<true>, cfg.num_sms * 4, 32 * WLONG_WARPS, s, a);
+      } else {
         pdl(k_ofold<false, true>, cfg.num_sms * 8, 128, s, a);
+        pdl(k_wlong<false>, cfg.num_sms * 4, 32 * WLONG_WARPS, s, a);
+      }
+      launches += 1;
     } else if (a.shadow_keys) {
       pdl(k_ofold<true, false>, cfg.num_sms * 8, 128, s, a);
     } else {
@@ -2217,17 +2223,20 @@ __global__ void __launch_bounds__(1024) k_oscan(FrameArgs a) {
 /* Links a fragment into sample px's list.  Node and touched-list slots come
  * from warp-aggregated allocations (one atomic per group of converged lanes,
  * not one per fragment on two shared counters); the fold sorts each list,
- * so the order of the slots does not matter. */
-__device__ __forceinline__ void push_fragment(const FrameArgs &a, uint32_t px, uint32_t order) {
+ * so the order of the slots does not matter.  Returns the node, 0xffffffff
+ * when the pool is full. */
+__device__ __forceinline__ uint32_t push_fragment(const FrameArgs &a, uint32_t px,
+                                                  uint32_t order) {
   const uint32_t node = warp_alloc1(&a.ctr->frag_count);
   if (node >= a.frag_cap) {
     atomicOr(&a.ctr->overflow, 16u);
-    return;
+    return 0xffffffffu;
   }
   const uint32_t prev = atomicExch(&a.frag_head[px], node);
   a.frags[node] = make_uint2(prev, order);
   if (prev == 0xffffffffu) /* first fragment of this sample */
     a.touched[warp_alloc1(&a.ctr->touched_count)] = px;
+  return node;
 }
 
 /* One (row, 32-sample chunk) item of a suffix record (nl: records queued):
@@ -2394,7 +2403,7 @@ __device__ __forceinline__ void wu_edge(const RasterRec &r, int e, WuLine &L) {
 /* The wireframe plot behind item `it` (the frame's wire-item numbering):
  * its record, edge and plot. */
 __device__ __forceinline__ bool wire_item(const FrameArgs &a, uint32_t it, uint32_t &rid,
-                                          WuLine &L, uint32_t &k) {
+                                          WuLine &L, uint32_t &k, uint32_t &base) {
   uint32_t nl = a.ctr->wire_count;
   if (nl > a.wlist_cap)
     nl = a.wlist_cap;
@@ -2412,7 +2421,8 @@ __device__ __forceinline__ bool wire_item(const FrameArgs &a, uint32_t it, uint3
   if (rid >= a.rec_cap)
     return false;
   const RasterRec r = a.rrec[rid];
-  k = it - a.wlist_items[lo];
+  base = a.wlist_items[lo];
+  k = it - base;
   for (int e = 0; e < 3; e++) {
     wu_edge(r, e, L);
     const uint32_t n = wu_plots(L);
@@ -2423,29 +2433,15 @@ __device__ __forceinline__ bool wire_item(const FrameArgs &a, uint32_t it, uint3
   return false;
 }
 
-/* Sort key of a fragment payload: (order, position among the record's
- * plots) for a line plot, (order, 0) for a filled record. */
-__device__ __forceinline__ unsigned long long frag_key(const FrameArgs &a, uint32_t v) {
-  if (!(v & FRAG_WIRE_BIT))
+/* Sort key of fragment node `node` with payload v: (order, 1 + position among
+ * the record's plots) for a line plot, (order, 0) for a filled record; a
+ * record is one or the other, so the low word tells them apart. */
+__device__ __forceinline__ unsigned long long frag_key(const FrameArgs &a, uint32_t node,
+                                                       uint32_t v) {
+  if (!a.wire || !(v & FRAG_WIRE_BIT)) /* a batch viewport without line plots may have any order */
     return (unsigned long long)v << 32;
-  const uint32_t it = v & ~FRAG_WIRE_BIT;
-  uint32_t nl = a.ctr->wire_count;
-  if (nl > a.wlist_cap)
-    nl = a.wlist_cap;
-  if (nl == 0u)
-    return ~0ull;
-  uint32_t lo = 0, hi = nl;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (a.wlist_items[mid] <= it)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  const uint32_t rid = a.wlist[lo];
-  if (rid >= a.rec_cap)
-    return ~0ull;
-  return ((unsigned long long)a.rrec[rid].order << 32) | (unsigned long long)(it - a.wlist_items[lo]);
+  const uint2 k = *reinterpret_cast<const uint2 *>(&a.wplots[node]);
+  return ((unsigned long long)k.x << 32) | (unsigned long long)k.y;
 }
 
 /* Queues the live wireframe records of the suffix with their plot counts. */
@@ -2487,13 +2483,16 @@ __global__ void __launch_bounds__(1024) k_wscan(FrameArgs a) {
 
 /* One line plot: in the framebuffer, coverage at least 0.004 and in front
  * of the opaque depth (or any depth when the suffix keeps every fragment)
- * gives a fragment. */
+ * gives a fragment, and all the fold needs of the plot goes into its WirePlot:
+ * the fold finding the record and the line again per fragment (a search of
+ * the queue for the key, another for the plot, the line's set-up and its row
+ * fold) took 605 of a 685 us 1280x720 frame of 40,448 triangles. */
 __device__ __forceinline__ void wplot_item(const FrameArgs &a, uint32_t it) {
   if (it >= FRAG_WIRE_BIT)
     return;
-  uint32_t rid, k;
+  uint32_t rid, k, base;
   WuLine L;
-  if (!wire_item(a, it, rid, L, k))
+  if (!wire_item(a, it, rid, L, k, base))
     return;
   int x, y;
   float z, cov;
@@ -2501,8 +2500,23 @@ __device__ __forceinline__ void wplot_item(const FrameArgs &a, uint32_t it) {
   if (x < 0 || x >= a.width || y < 0 || y >= a.height || cov < 0.004f)
     return;
   const uint32_t px = (uint32_t)y * (uint32_t)a.width + (uint32_t)x;
-  if (a.ordered_keep_all || z < a.depth[px])
-    push_fragment(a, px, FRAG_WIRE_BIT | it);
+  if (!(a.ordered_keep_all || z < a.depth[px]))
+    return;
+  const uint32_t node = push_fragment(a, px, FRAG_WIRE_BIT);
+  if (node == 0xffffffffu)
+    return;
+  const ShadeRec s = a.srec[rid];
+  WirePlot w;
+  w.order = a.rrec[rid].order;
+  w.k1 = 1u + (it - base);
+  w.z = z;
+  w.cov = cov;
+  for (int c = 0; c < 3; c++) {
+    const float v = s.col[c] > 1.0f ? 1.0f : s.col[c];
+    w.src[c] = (float)(uint8_t)x86_f2i(v * 255.0f) / 255.0f;
+  }
+  w.draw = s.draw;
+  a.wplots[node] = w;
 }
 
 __global__ void __launch_bounds__(256) k_wplot(FrameArgs a) {
@@ -2536,47 +2550,40 @@ struct OFold {
   bool cur_nw;
 };
 
-/* A fragment of draw di follows: when the draw changes, a finished
- * depth-write-off draw's depth is undone (cpu_backend.c:575-580) and a new
- * one's saved (:536-544). */
-__device__ __forceinline__ void ofold_enter_draw(OFold &st, uint32_t di, const DrawRec &d) {
+/* A fragment of draw di (with `flags`) follows: when the draw changes, a
+ * finished depth-write-off draw's depth is undone (cpu_backend.c:575-580) and a
+ * new one's saved (:536-544). */
+__device__ __forceinline__ void ofold_enter_draw(OFold &st, uint32_t di, uint32_t flags) {
   if (di != st.cur) {
     if (st.cur_nw)
       st.depth = st.saved;
     st.cur = di;
-    st.cur_nw = (d.flags & DF_NO_DEPTH_WRITE) != 0;
+    st.cur_nw = (flags & DF_NO_DEPTH_WRITE) != 0;
     if (st.cur_nw)
       st.saved = st.depth;
   }
 }
 
-/* Applies line plot `it` at its sample: aa_plot (rasterizer.c:687-729) on
- * the sample's HDR colour, depth and ID. */
-__device__ __forceinline__ void ofold_wire(const FrameArgs &a, OFold &st, uint32_t it) {
-  uint32_t rid, k;
-  WuLine L;
-  if (!wire_item(a, it, rid, L, k))
+/* Applies line plot w of draw di: aa_plot (rasterizer.c:687-729) on the
+ * sample's HDR colour, depth and ID. */
+__device__ __forceinline__ void ofold_plot(OFold &st, const WirePlot &w, uint32_t di,
+                                           uint32_t flags, uint32_t id) {
+  ofold_enter_draw(st, di, flags);
+  if (!(flags & DF_NO_DEPTH_TEST) && w.z >= st.depth)
     return;
-  const ShadeRec s = a.srec[rid];
-  const uint32_t di = s.draw < a.draw_count ? s.draw : 0;
-  const DrawRec &d = a.draws[di];
-  ofold_enter_draw(st, di, d);
-  int px, py;
-  float z, cov;
-  wu_plot(L, k, px, py, z, cov);
-  if (!(d.flags & DF_NO_DEPTH_TEST) && z >= st.depth)
-    return;
-  const float inv = 1.0f - cov;
-  for (int c = 0; c < 3; c++) {
-    /* the line colour as the reference's byte (rasterizer.c:1226-1228) */
-    const float v = s.col[c] > 1.0f ? 1.0f : s.col[c];
-    const float src = (float)(uint8_t)x86_f2i(v * 255.0f) / 255.0f;
-    st.hdr[c] = src * cov + st.hdr[c] * inv;
+  const float inv = 1.0f - w.cov;
+  for (int c = 0; c < 3; c++)
+    st.hdr[c] = w.src[c] * w.cov + st.hdr[c] * inv;
+  if (w.cov > 0.5f) {
+    st.depth = w.z;
+    st.id = id;
   }
-  if (cov > 0.5f) {
-    st.depth = z;
-    st.id = d.object_id;
-  }
+}
+
+__device__ __forceinline__ void ofold_wire(const FrameArgs &a, OFold &st, uint32_t node) {
+  const WirePlot w = a.wplots[node];
+  const uint32_t di = w.draw < a.draw_count ? w.draw : 0;
+  ofold_plot(st, w, di, a.draws[di].flags, a.draws[di].object_id);
 }
 
 /* Applies the fragment of submission order `order` at sample (x, y). */
@@ -2590,7 +2597,7 @@ __device__ __forceinline__ void ofold_fragment(const FrameArgs &a, OFold &st, in
   const ShadeRec s = a.srec[rid];
   const uint32_t di = s.draw < a.draw_count ? s.draw : 0;
   const DrawRec &d = a.draws[di];
-  ofold_enter_draw(st, di, d);
+  ofold_enter_draw(st, di, d.flags);
   const bool dtest = !(d.flags & DF_NO_DEPTH_TEST);
   const int jr = y - (int)r.y0, kc = x - (int)r.x0;
   if (r.y1 & REC_FLAT_BIT) { /* rasterize_filled_triangle, rasterizer.c:1000-1083 */
@@ -2715,38 +2722,22 @@ __device__ __noinline__ void heapsort_keys(ulonglong2 *h, uint32_t n) {
 /* Each touched sample folds its fragments in submission order.  Up to
  * ORDERED_MAX_FRAGS are gathered and insertion-sorted in registers; a
  * longer list is copied with its keys into the fold's scratch and heapsorted
- * there (keys are distinct: a record covers a sample once, a line plot is
- * one item).  WIRE: the frame has line
- * plots, whose payloads sort by frag_key (a triangle's plots in the
- * reference's drawing order after the triangles before it). */
-template <bool WIRE>
-__device__ __forceinline__ unsigned long long ofold_key(const FrameArgs &a, uint32_t v) {
-  return (WIRE && a.wire) ? frag_key(a, v) : (unsigned long long)v;
-}
-
+ * there, or in a wireframe frame left to a warp of its own (keys are
+ * distinct: a record covers a sample once, a line plot is one item).  WIRE: the launch has line plots, which sort by frag_key (a
+ * triangle's plots in the reference's drawing order after the triangles
+ * before it); fragments then travel as (key, node), others as their order. */
 template <bool SH, bool WIRE>
 __device__ __forceinline__ void ofold_apply(const FrameArgs &a, OFold &st, int x, int y,
-                                            uint32_t v) {
-  if (WIRE && a.wire && (v & FRAG_WIRE_BIT))
-    ofold_wire(a, st, v & ~FRAG_WIRE_BIT);
+                                            unsigned long long key, uint32_t v) {
+  if (WIRE && (uint32_t)key != 0u)
+    ofold_wire(a, st, v);
   else
-    ofold_fragment<SH>(a, st, x, y, v);
+    ofold_fragment<SH>(a, st, x, y, WIRE ? (uint32_t)(key >> 32) : v);
 }
 
-template <bool SH, bool WIRE>
-__device__ __forceinline__ void ofold_item(const FrameArgs &a, uint32_t i) {
-  const uint32_t px = a.touched[i];
-  const uint32_t head = a.frag_head[px];
-  uint32_t ord[ORDERED_MAX_FRAGS];
-  uint32_t cnt = 0, total = 0;
-  for (uint32_t node = head; node != 0xffffffffu && node < a.frag_cap; node = a.frags[node].x) {
-    if (cnt < ORDERED_MAX_FRAGS)
-      ord[cnt++] = a.frags[node].y;
-    if (++total > a.frag_cap)
-      break;
-  }
-  const int x = (int)(px % (uint32_t)a.width), y = (int)(px / (uint32_t)a.width);
-  OFold st;
+/* The sample's state before its suffix. */
+__device__ __forceinline__ void ofold_begin(const FrameArgs &a, OFold &st, uint32_t px, int x,
+                                            int y) {
   if (a.keys[px] != KEY_EMPTY) {
     const float4 h = a.hdr[px];
     st.hdr[0] = h.x;
@@ -2764,57 +2755,12 @@ __device__ __forceinline__ void ofold_item(const FrameArgs &a, uint32_t i) {
   st.saved = st.depth;
   st.cur = 0xffffffffu;
   st.cur_nw = false;
-  if (total <= ORDERED_MAX_FRAGS) {
-    if (WIRE && a.wire) { /* keys computed once: a plot's key takes a search */
-      unsigned long long key[WIRE ? ORDERED_MAX_FRAGS : 1];
-      for (uint32_t k = 0; k < cnt; k++)
-        key[k] = frag_key(a, ord[k]);
-      for (uint32_t k = 1; k < cnt; k++) {
-        const uint32_t v = ord[k];
-        const unsigned long long kv = key[k];
-        uint32_t j = k;
-        while (j > 0 && key[j - 1] > kv) {
-          ord[j] = ord[j - 1];
-          key[j] = key[j - 1];
-          j--;
-        }
-        ord[j] = v;
-        key[j] = kv;
-      }
-    } else {
-      for (uint32_t k = 1; k < cnt; k++) { /* submission order */
-        const uint32_t v = ord[k];
-        uint32_t j = k;
-        while (j > 0 && ord[j - 1] > v) {
-          ord[j] = ord[j - 1];
-          j--;
-        }
-        ord[j] = v;
-      }
-    }
-    for (uint32_t k = 0; k < cnt; k++)
-      ofold_apply<SH, WIRE>(a, st, x, y, ord[k]);
-  } else {
-    /* a long list: its (key, payload) pairs heapsorted in the scratch */
-    const uint32_t base = atomicAdd(a.oscratch_count, total);
-    if (!a.oscratch || (unsigned long long)base + total > a.oscratch_cap) {
-      atomicOr(&a.ctr->overflow, 16u); /* unreachable: the scratch holds the fragment pool */
-      return;
-    }
-    ulonglong2 *sc = a.oscratch + base;
-    uint32_t m = 0;
-    for (uint32_t node = head; node != 0xffffffffu && node < a.frag_cap && m < total;
-         node = a.frags[node].x) {
-      const uint32_t v = a.frags[node].y;
-      sc[m++] = make_ulonglong2(ofold_key<WIRE>(a, v), (unsigned long long)v);
-    }
-    heapsort_keys(sc, m);
-    for (uint32_t k = 0; k < m; k++)
-      ofold_apply<SH, WIRE>(a, st, x, y, (uint32_t)sc[k].y);
-  }
+}
+
+/* Writes the composited sample: mop_sw_hdr_resolve (rasterizer.c:2776-2803). */
+__device__ __forceinline__ void ofold_end(const FrameArgs &a, OFold &st, uint32_t px) {
   if (st.cur_nw)
     st.depth = st.saved;
-  /* mop_sw_hdr_resolve (rasterizer.c:2776-2803) of the composited sample */
   if (st.id == 0u)
     a.pre[px] = make_uchar4(x86_f2u8(fminf(st.hdr[0], 1.0f) * 255.0f + 0.5f),
                             x86_f2u8(fminf(st.hdr[1], 1.0f) * 255.0f + 0.5f),
@@ -2828,11 +2774,181 @@ __device__ __forceinline__ void ofold_item(const FrameArgs &a, uint32_t i) {
 }
 
 template <bool SH, bool WIRE>
+__device__ __forceinline__ void ofold_item(const FrameArgs &a, uint32_t i) {
+  constexpr uint32_t MAX = WIRE ? WIRE_THREAD_FRAGS : ORDERED_MAX_FRAGS;
+  const uint32_t px = a.touched[i];
+  const uint32_t head = a.frag_head[px];
+  uint32_t ord[MAX];                      /* order; WIRE: node */
+  unsigned long long key[WIRE ? MAX : 1]; /* WIRE: sort keys   */
+  uint32_t cnt = 0, total = 0;
+  for (uint32_t node = head; node != 0xffffffffu && node < a.frag_cap;) {
+    const uint2 f = a.frags[node];
+    if (cnt < MAX) {
+      if (WIRE)
+        key[cnt] = frag_key(a, node, f.y);
+      ord[cnt++] = WIRE ? node : f.y;
+    }
+    if (++total > a.frag_cap)
+      break;
+    node = f.x;
+  }
+  const int x = (int)(px % (uint32_t)a.width), y = (int)(px / (uint32_t)a.width);
+  OFold st;
+  if (total <= MAX) {
+    ofold_begin(a, st, px, x, y);
+    for (uint32_t k = 1; k < cnt; k++) { /* submission order */
+      const uint32_t v = ord[k];
+      const unsigned long long kv = WIRE ? key[WIRE ? k : 0] : (unsigned long long)v;
+      uint32_t j = k;
+      while (j > 0 && (WIRE ? key[WIRE ? j - 1 : 0] : (unsigned long long)ord[j - 1]) > kv) {
+        ord[j] = ord[j - 1];
+        if (WIRE)
+          key[j] = key[j - 1];
+        j--;
+      }
+      ord[j] = v;
+      if (WIRE)
+        key[j] = kv;
+    }
+    for (uint32_t k = 0; k < cnt; k++)
+      ofold_apply<SH, WIRE>(a, st, x, y, key[WIRE ? k : 0], ord[k]);
+  } else {
+    /* a long list: its (key, payload) pairs in the scratch */
+    const uint32_t base = atomicAdd(a.oscratch_count, total);
+    if (!a.oscratch || (unsigned long long)base + total > a.oscratch_cap) {
+      atomicOr(&a.ctr->overflow, 16u); /* unreachable: the scratch holds the fragment pool */
+      return;
+    }
+    ulonglong2 *sc = a.oscratch + base;
+    uint32_t m = 0;
+    for (uint32_t node = head; node != 0xffffffffu && node < a.frag_cap && m < total;) {
+      const uint2 f = a.frags[node];
+      sc[m++] = WIRE ? make_ulonglong2(frag_key(a, node, f.y), (unsigned long long)node)
+                     : make_ulonglong2((unsigned long long)f.y, (unsigned long long)f.y);
+      node = f.x;
+    }
+    if (WIRE) { /* left to wlong_item: the list's place and length ride in buffers whose
+                   values for this sample are spent (head, unused hdr component); the
+                   queue takes the shading list's place */
+      a.frag_head[px] = base;
+      a.hdr[px].w = __uint_as_float(m);
+      a.shade_list[warp_alloc1(&a.ctr->wlong_count)] = px;
+      return;
+    }
+    ofold_begin(a, st, px, x, y);
+    heapsort_keys(sc, m);
+    for (uint32_t k = 0; k < m; k++)
+      ofold_apply<SH, WIRE>(a, st, x, y, sc[k].x, (uint32_t)sc[k].y);
+  }
+  ofold_end(a, st, px);
+}
+
+template <bool SH, bool WIRE>
 __global__ void __launch_bounds__(128) k_ofold(FrameArgs a) {
   pdl_wait();
   const uint32_t n = a.ctr->touched_count;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     ofold_item<SH, WIRE>(a, i);
+}
+
+/* Long lists of a wireframe frame, a warp per sample.  Wireframes pile
+ * hundreds of plots on the samples of a distant mesh, and a frame's fold
+ * took as long as its longest list: a thread that heapsorted and folded it
+ * alone, one dependent load after another (250 us at 1280x720, 40,448
+ * triangles, where this kernel and the threads' fold together take 143).  The warp sorts up to
+ * WLONG_SORT pairs bitonically in shared memory (longer lists are
+ * heapsorted by lane 0), then fetches 32 plots at a time, a lane each, and
+ * all lanes fold them in order from shared memory, redundantly. */
+#define WLONG_SORT 512
+
+struct WLongSmem {
+  unsigned long long key[WLONG_SORT];
+  uint32_t node[WLONG_SORT];
+  WirePlot plot[32];
+  uint2 draw[32]; /* flags, object id */
+};
+
+__device__ __forceinline__ void wlong_sort(WLongSmem &sm, ulonglong2 *sc, uint32_t n,
+                                           uint32_t lane) {
+  uint32_t P = 64;
+  while (P < n)
+    P <<= 1;
+  for (uint32_t i = lane; i < P; i += 32u) {
+    const ulonglong2 e = i < n ? sc[i] : make_ulonglong2(~0ull, 0ull);
+    sm.key[i] = e.x;
+    sm.node[i] = (uint32_t)e.y;
+  }
+  __syncwarp();
+  for (uint32_t size = 2; size <= P; size <<= 1)
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      for (uint32_t t = lane; t < P / 2u; t += 32u) {
+        const uint32_t i = 2u * t - (t & (stride - 1u)), j = i + stride;
+        const unsigned long long ki = sm.key[i], kj = sm.key[j];
+        if ((ki > kj) == ((i & size) == 0u)) {
+          sm.key[i] = kj;
+          sm.key[j] = ki;
+          const uint32_t ni = sm.node[i];
+          sm.node[i] = sm.node[j];
+          sm.node[j] = ni;
+        }
+      }
+      __syncwarp();
+    }
+}
+
+/* Sample shade_list[q], by one whole warp. */
+template <bool SH>
+__device__ __forceinline__ void wlong_item(const FrameArgs &a, uint32_t q, WLongSmem &sm) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t px = a.shade_list[q];
+  const uint32_t n = __float_as_uint(a.hdr[px].w);
+  ulonglong2 *sc = a.oscratch + a.frag_head[px];
+  const int x = (int)(px % (uint32_t)a.width), y = (int)(px / (uint32_t)a.width);
+  const bool in_smem = n <= WLONG_SORT;
+  if (in_smem)
+    wlong_sort(sm, sc, n, lane);
+  else if (lane == 0)
+    heapsort_keys(sc, n);
+  __syncwarp();
+  OFold st;
+  ofold_begin(a, st, px, x, y);
+  for (uint32_t b = 0; b < n; b += 32u) {
+    const uint32_t i = b + lane;
+    if (i < n) {
+      const unsigned long long key = in_smem ? sm.key[i] : sc[i].x;
+      if ((uint32_t)key != 0u) {
+        const WirePlot w = a.wplots[in_smem ? sm.node[i] : (uint32_t)sc[i].y];
+        sm.plot[lane] = w;
+        const DrawRec &d = a.draws[w.draw < a.draw_count ? w.draw : 0];
+        sm.draw[lane] = make_uint2(d.flags, d.object_id);
+      } else { /* a filled record's fragment */
+        sm.plot[lane].order = (uint32_t)(key >> 32);
+        sm.plot[lane].k1 = 0u;
+      }
+    }
+    __syncwarp();
+    const uint32_t m = min(32u, n - b);
+    for (uint32_t j = 0; j < m; j++) {
+      const WirePlot w = sm.plot[j];
+      if (w.k1 == 0u) {
+        ofold_fragment<SH>(a, st, x, y, w.order);
+        continue;
+      }
+      const uint2 d = sm.draw[j];
+      ofold_plot(st, w, w.draw < a.draw_count ? w.draw : 0, d.x, d.y);
+    }
+    __syncwarp(); /* the plots are read before the next 32 replace them */
+  }
+  if (lane == 0)
+    ofold_end(a, st, px);
+}
+
+template <bool SH> __global__ void __launch_bounds__(32 * WLONG_WARPS) k_wlong(FrameArgs a) {
+  pdl_wait();
+  __shared__ WLongSmem sm[WLONG_WARPS];
+  const uint32_t n = a.ctr->wlong_count, warp = threadIdx.x >> 5;
+  for (uint32_t q = blockIdx.x * WLONG_WARPS + warp; q < n; q += gridDim.x * WLONG_WARPS)
+    wlong_item<SH>(a, q, sm[warp]);
 }
 
 /* ========================================================================
@@ -3103,6 +3219,7 @@ __global__ void __launch_bounds__(256) k_batch_prepare(BatchArgs b) {
     a.wire = (int)s_wire;
     a.wlist = a.wlist_items = nullptr;
     a.wlist_cap = 0u;
+    a.wplots = nullptr;
     a.oscratch = b.oscratch;
     a.oscratch_count = b.oscratch_count;
     a.oscratch_cap = (uint32_t)(b.frag_pool < 0xffffffffull ? b.frag_pool : 0xffffffffull);
@@ -3220,6 +3337,7 @@ __global__ void __launch_bounds__(256) k_batch_alloc(BatchArgs b) {
         a.frags = b.frags + off[5];
         a.frag_cap = (uint32_t)(need[5] < 0xfffffff0ull ? need[5] : 0xfffffff0ull);
         if (a.wire) {
+          a.wplots = b.wplots + off[5];
           a.wlist = b.wlist + off[6];
           a.wlist_items = b.wlist_items + off[6];
           a.wlist_cap = (uint32_t)need[6];
@@ -3240,7 +3358,7 @@ __global__ void __launch_bounds__(256) k_batch_alloc(BatchArgs b) {
 }
 
 enum { ST_VERTEX, ST_SETUP, ST_CLIP, ST_RSMALL, ST_RLARGE, ST_SHADE, ST_RESOLVE, ST_OCOUNT,
-       ST_ORASTER, ST_OFOLD, ST_WCOUNT, ST_WPLOT };
+       ST_ORASTER, ST_OFOLD, ST_WCOUNT, ST_WPLOT, ST_WLONG };
 
 template <int ST> __device__ __forceinline__ uint32_t stage_count(const FrameArgs &a) {
   switch (ST) {
@@ -3266,6 +3384,8 @@ template <int ST> __device__ __forceinline__ uint32_t stage_count(const FrameArg
     return a.hdr && a.wire && a.total_tris ? ordered_record_items(a) : 0u;
   case ST_WPLOT:
     return a.hdr && a.wire ? a.ctr->wire_items : 0u;
+  case ST_WLONG:
+    return a.hdr ? a.ctr->wlong_count : 0u;
   default: /* ST_RESOLVE: chunks of 256 x RESOLVE_PER_THREAD samples */
     return ((uint32_t)a.width * (uint32_t)a.height + 256u * RESOLVE_PER_THREAD - 1u) /
            (256u * RESOLVE_PER_THREAD);
@@ -3442,6 +3562,20 @@ __global__ void __launch_bounds__(128) k_b_ofold(const FrameArgs *__restrict__ f
   }
 }
 
+template <bool SH>
+__global__ void __launch_bounds__(32 * WLONG_WARPS) k_b_wlong(const FrameArgs *__restrict__ fr,
+                                                              uint32_t nv) {
+  __shared__ uint32_t s_pre[MOPCUDA_MAX_VIEWS + 1];
+  __shared__ WLongSmem sm[WLONG_WARPS];
+  const uint32_t total = views_prefix<ST_WLONG>(fr, nv, s_pre), warp = threadIdx.x >> 5;
+  uint32_t v = 0;
+  for (uint32_t q = blockIdx.x * WLONG_WARPS + warp; q < total; q += gridDim.x * WLONG_WARPS) {
+    while (s_pre[v + 1] <= q)
+      v++;
+    wlong_item<SH>(fr[v], q - s_pre[v], sm[warp]);
+  }
+}
+
 template <int SF>
 __device__ __forceinline__ uint32_t post_tiles_of(const PostArgs &p) {
   const uint32_t pw = (uint32_t)(p.width / SF), ph = (uint32_t)(p.height / SF);
@@ -3551,10 +3685,14 @@ int mopcuda_launch_batch(const BatchArgs &b, const PostArgs *posts, const uint32
         k_b_wscan<<<nv, 1024, 0, s>>>(fr);
         k_b_wplot<<<sms * 8, 256, 0, s>>>(fr, nv);
         launches += 3;
-        if (shadows)
+        if (shadows) {
           k_b_ofold<true, true><<<sms * 8, 128, 0, s>>>(fr, nv);
-        else
+          k_b_wlong<true><<<sms * 4, 32 * WLONG_WARPS, 0, s>>>(fr, nv);
+        } else {
           k_b_ofold<false, true><<<sms * 8, 128, 0, s>>>(fr, nv);
+          k_b_wlong<false><<<sms * 4, 32 * WLONG_WARPS, 0, s>>>(fr, nv);
+        }
+        launches += 1;
       } else if (shadows) {
         k_b_ofold<true, false><<<sms * 8, 128, 0, s>>>(fr, nv);
       } else {

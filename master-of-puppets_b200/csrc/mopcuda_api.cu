@@ -156,7 +156,7 @@ extern "C" void mopcuda_device_destroy(MopCudaDevice *d) {
                         &d->large_items,
                         &d->shade_list, &d->counters, &d->pick_xy,     &d->pick_out,
                         &d->deform_params, &d->hdr, &d->frag_head, &d->frags, &d->touched,
-                        &d->olist, &d->olist_items, &d->wlist, &d->wlist_items, &d->oscratch, &d->sh_map[0], &d->sh_map[1], &d->sh_d_draws,
+                        &d->olist, &d->olist_items, &d->wlist, &d->wlist_items, &d->wplots, &d->oscratch, &d->sh_map[0], &d->sh_map[1], &d->sh_d_draws,
                         &d->sh_recs, &d->sh_items, &d->sh_ctr, &d->env, &d->ibl_tab};
   for (DevArena *a : arenas)
     a->release();
@@ -1121,6 +1121,7 @@ static int launch_frame(MopCudaDevice *d) {
                     (unsigned long long)T);
       rc |= d->wlist.ensure(4ull * ocap);
       rc |= d->wlist_items.ensure(4ull * ocap);
+      rc |= d->wplots.ensure(sizeof(WirePlot) * (size_t)fcap);
     }
   }
   if (rc)
@@ -1219,6 +1220,7 @@ static int launch_frame(MopCudaDevice *d) {
       a.wlist = d->wlist.as<uint32_t>();
       a.wlist_items = d->wlist_items.as<uint32_t>();
       a.wlist_cap = ocap;
+      a.wplots = d->wplots.as<WirePlot>();
     }
   }
 

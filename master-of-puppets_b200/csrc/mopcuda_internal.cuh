@@ -114,10 +114,20 @@ struct __align__(16) RasterRec {
  * kernel takes it: its box is empty), w0/dx/dy hold the screen x, y and z of
  * its three vertices. */
 #define REC_WIRE_X1 0x8000u
-/* Fragment payloads of wireframe frames: bit 31 set marks a line plot, the
- * rest its item index (the frame's triangle count stays below 2^26, so
- * triangle orders keep bit 31 clear). */
+/* Fragment payloads of wireframe frames: bit 31 set marks a line plot (its
+ * data is the fragment's WirePlot; the frame's triangle count stays below
+ * 2^26, so triangle orders keep bit 31 clear). */
 #define FRAG_WIRE_BIT 0x80000000u
+
+/* A line plot as the fold needs it, written beside its fragment node. */
+struct __align__(16) WirePlot {
+  uint32_t order;  /* of its triangle */
+  uint32_t k1;     /* 1 + position among the triangle's plots */
+  float z, cov;
+  float src[3];    /* the line colour, a byte / 255 (rasterizer.c:1226-1228) */
+  uint32_t draw;
+};
+static_assert(sizeof(WirePlot) == 32, "one sector per plot");
 
 /* Per fan-triangle shading record, 16 bytes. */
 struct __align__(16) ShadeRec {
@@ -147,7 +157,8 @@ struct alignas(8) Counters {
   uint32_t frag_count, touched_count, olist_count, olist_items;
   uint32_t wire_count, wire_items; /* wireframe records queued, their plots */
   uint32_t scratch_count;          /* sort-scratch entries taken by long lists */
-  uint32_t pad[2];
+  uint32_t wlong_count;            /* samples of wireframe frames with a long list */
+  uint32_t pad;
 };
 /* arrays of counters (one per viewport) keep the 64-bit pair aligned */
 static_assert(sizeof(Counters) % 8 == 0 && offsetof(Counters, large_items) % 8 == 0,
@@ -156,6 +167,9 @@ static_assert(sizeof(Counters) % 8 == 0 && offsetof(Counters, large_items) % 8 =
 /* Blended fragments of one sample sorted in registers; a sample with more
  * sorts its list in the fold's global scratch (heapsort). */
 #define ORDERED_MAX_FRAGS 48
+/* In a wireframe frame a thread folds lists of up to this many fragments;
+ * longer ones are folded by a warp each. */
+#define WIRE_THREAD_FRAGS 24
 
 /* Records whose clamped bbox exceeds these bounds are rasterised as
  * (row, RASTER_CHUNK-sample) items spread over many threads; smaller ones
@@ -242,6 +256,7 @@ struct FrameArgs {
   uint32_t *wlist, *wlist_items;
   uint32_t wlist_cap;
   int wire;
+  WirePlot *wplots; /* per fragment node: its line plot (frag_cap entries) */
   /* sort scratch of the fold for lists longer than ORDERED_MAX_FRAGS:
    * (key, payload) pairs, oscratch_cap entries (at least the fragment pool,
    * so it cannot run out), taken from *oscratch_count */
@@ -475,6 +490,7 @@ struct BatchArgs {
   unsigned long long olist_pool;
   uint32_t *wlist, *wlist_items; /* wireframe-record lists (null: no wireframe draws) */
   unsigned long long wlist_pool;
+  WirePlot *wplots;              /* frag_pool entries, at the fragments' offsets */
   ulonglong2 *oscratch;          /* the fold's sort scratch, frag_pool entries, shared */
   uint32_t *oscratch_count;      /* by the launch's viewports through one counter */
   unsigned long long samples; /* samples of the launch (frag_head's length) */
