@@ -199,7 +199,7 @@ struct MopCudaDevice {
   bool ibl_on = false;
   /* frame arenas */
   DevArena d_draws, d_lights, clip, world, normal, color, rrec, srec, clipq,
-      large_list, large_items, shade_list, counters, pick_xy, pick_out;
+      large_lists, chunk_w, shade_list, counters, pick_xy, pick_out;
   /* visibility keys: two buffers in turn, a frame's shading pass clearing the
    * one the next frame uses; keys_clean[i] = samples of buffer i known clear */
   DevArena keys[2];

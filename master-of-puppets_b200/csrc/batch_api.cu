@@ -336,7 +336,7 @@ void LaunchCore::release() {
     sync(10000);
   DevArena *arenas[] = {&d_views, &d_frames, &d_view_draws, &d_ctr, &d_status, &d_posts,
                         &d_post_views, &d_draws, &d_scenes, &clip, &world, &normal, &color,
-                        &rrec, &srec, &clipq, &large_list, &large_items, &keys, &shade_list,
+                        &rrec, &srec, &clipq, &large_list, &large_items, &wide_list, &wide_items, &large_off, &chunk_w, &keys, &shade_list,
                         &pre, &out, &depth, &ids, &presented, &hdr, &frag_head, &touched,
                         &frags, &olist, &olist_items, &wlist, &wlist_items, &wplots, &oscratch};
   for (DevArena *a : arenas)
@@ -367,7 +367,7 @@ void LaunchCore::trim() {
   if (stream)
     sync(10000);
   DevArena *arenas[] = {&clip,       &world, &normal,  &color,      &rrec,      &srec,
-                        &clipq,      &large_list, &large_items, &keys, &shade_list, &pre,
+                        &clipq,      &large_list, &large_items, &wide_list, &wide_items, &large_off, &chunk_w, &keys, &shade_list, &pre,
                         &out,        &depth, &ids,     &presented,  &hdr,       &frag_head,
                         &touched,    &frags, &olist,   &olist_items, &wlist, &wlist_items,
                         &wplots,     &oscratch};
@@ -380,7 +380,8 @@ void LaunchCore::trim() {
 uint64_t LaunchCore::device_bytes() const {
   const DevArena *arenas[] = {&d_views, &d_frames, &d_view_draws, &d_ctr, &d_status, &d_posts,
                               &d_post_views, &d_draws, &d_scenes, &clip, &world, &normal, &color,
-                              &rrec, &srec, &clipq, &large_list, &large_items, &keys,
+                              &rrec, &srec, &clipq, &large_list, &large_items, &wide_list, &wide_items, &large_off,
+                              &chunk_w, &keys,
                               &shade_list, &pre, &out, &depth, &ids, &presented, &hdr,
                               &frag_head, &touched, &frags, &olist, &olist_items, &wlist,
                               &wlist_items, &wplots, &oscratch};
@@ -448,6 +449,7 @@ int LaunchCore::set_layout(const MopCudaView *views, const uint32_t *scene_of,
   const unsigned long long sa = std::max(so, sample_floor), pa = std::max(po, pixel_floor);
   rc |= keys.ensure(8ull * sa);
   rc |= shade_list.ensure(4ull * sa);
+  rc |= chunk_w.ensure(16ull * chunk_entries(sa));
   rc |= pre.ensure(4ull * sa);
   rc |= out.ensure(4ull * sa);
   rc |= depth.ensure(4ull * sa);
@@ -510,14 +512,19 @@ static int size_pools(LaunchCore *b, unsigned long long vneed, unsigned long lon
   rc |= b->clipq.ensure(4ull * cneed);
   rc |= b->large_list.ensure(4ull * lneed);
   rc |= b->large_items.ensure(4ull * lneed);
+  rc |= b->wide_list.ensure(4ull * lneed);
+  rc |= b->wide_items.ensure(4ull * lneed);
+  rc |= b->large_off.ensure(4ull * rneed);
   if (rc)
     return MOPCUDA_ENOMEM;
   auto cap = [](const DevArena &a, size_t el) { return (unsigned long long)(a.cap / el); };
   b->vertex_pool = std::min(std::min(cap(b->clip, 16), cap(b->world, 16)),
                             std::min(cap(b->normal, 16), cap(b->color, 16)));
-  b->rec_pool = std::min(cap(b->rrec, sizeof(RasterRec)), cap(b->srec, sizeof(ShadeRec)));
+  b->rec_pool = std::min(std::min(cap(b->rrec, sizeof(RasterRec)), cap(b->srec, sizeof(ShadeRec))),
+                         cap(b->large_off, 4));
   b->clip_pool = cap(b->clipq, 4);
-  b->large_pool = std::min(cap(b->large_list, 4), cap(b->large_items, 4));
+  b->large_pool = std::min(std::min(cap(b->large_list, 4), cap(b->large_items, 4)),
+                           std::min(cap(b->wide_list, 4), cap(b->wide_items, 4)));
   return MOPCUDA_OK;
 }
 
@@ -746,7 +753,11 @@ int LaunchCore::enqueue(int parts) {
   a.clip_pool = clip_pool;
   a.large_list = large_list.as<uint32_t>();
   a.large_items = large_items.as<uint32_t>();
+  a.wide_list = wide_list.as<uint32_t>();
+  a.wide_items = wide_items.as<uint32_t>();
   a.large_pool = large_pool;
+  a.large_off = large_off.as<uint32_t>();
+  a.chunk_w = chunk_w.as<float4>();
   a.keys = keys.as<unsigned long long>();
   a.shade_list = shade_list.as<uint32_t>();
   a.pre = pre.as<uchar4>();

@@ -94,7 +94,8 @@ struct LaunchCore {
       d_scenes;
   HostArena h_views, h_draws, h_scenes, h_status;
   /* work pools */
-  DevArena clip, world, normal, color, rrec, srec, clipq, large_list, large_items;
+  DevArena clip, world, normal, color, rrec, srec, clipq, large_list, large_items,
+      wide_list, wide_items, large_off, chunk_w;
   unsigned long long vertex_pool = 0, rec_pool = 0, clip_pool = 0, large_pool = 0;
   uint32_t fan_num = 1, large_num = 1;
   /* pool sizes below which stage() does not go (a server sizes its slots

@@ -70,6 +70,19 @@ MOPCUDA_HD float fold_fadd(float a, float b) {
 #endif
 }
 
+/* A whole number of steps j with 0 <= j <= num / den, at most one short of it
+ * (0 <= num, 1 <= den, both below 2^24, so exact in single precision): the
+ * quotient's relative error, at most 2^-21 through the approximate division,
+ * is taken off before truncating.  A jump may stop short of its binade's edge:
+ * the explicit steps that follow any jump cover the rest. */
+MOPCUDA_HD int32_t fold_room(int32_t num, int32_t den) {
+#if defined(__CUDA_ARCH__)
+  return (int32_t)(__fdividef((float)num, (float)den) * 0.9999990f);
+#else
+  return (int32_t)(((float)num / (float)den) * 0.9999990f);
+#endif
+}
+
 #define FOLD_SERIAL_MAX 16
 
 /* The binade-skipping path of fold_add for k > FOLD_SERIAL_MAX (kept out of
@@ -108,7 +121,7 @@ MOPCUDA_HD_SLOW float fold_add_long(float w, float d, int k) {
     int32_t q = n3 - n2; /* steady increment of the magnitude */
     if (q == 0)
       return w3; /* the increment rounds away: w is a fixed point */
-    int32_t room = q > 0 ? (top - n3) / q : (n3 - lo) / (-q);
+    int32_t room = q > 0 ? fold_room(top - n3, q) : fold_room(n3 - lo, -q);
     int32_t j = room < k ? room : k;
     if (j <= 0)
       continue;
@@ -117,6 +130,71 @@ MOPCUDA_HD_SLOW float fold_add_long(float w, float d, int k) {
     k -= j;
   }
   return w;
+}
+
+/* One round of fold_add_long on (w, k), k > 0: up to three explicit steps and
+ * the jump they allow.  Straight-line, so that rounds of several folds
+ * interleave. */
+MOPCUDA_HD void fold_round(float *w, float d, int *k) {
+  const float w0 = *w;
+  const float w1 = fold_fadd(w0, d), w2 = fold_fadd(w1, d), w3 = fold_fadd(w2, d);
+  if (*k <= 3) {
+    *w = *k == 1 ? w1 : (*k == 2 ? w2 : w3);
+    *k = 0;
+    return;
+  }
+  *w = w3;
+  *k -= 3;
+  const uint32_t b1 = fold_bits(w1), b2 = fold_bits(w2), b3 = fold_bits(w3);
+  const uint32_t hi = b3 & 0xff800000u, ex = (hi >> 23) & 0xffu;
+  if (ex == 0xffu) { /* inf / NaN + finite d is stable */
+    *k = 0;
+    return;
+  }
+  const int32_t n2 = (int32_t)((b2 & 0x007fffffu) | 0x00800000u);
+  const int32_t n3 = (int32_t)((b3 & 0x007fffffu) | 0x00800000u);
+  const int32_t lo = 0x00800001, top = 0x00ffffff;
+  if ((b1 & 0xff800000u) != hi || (b2 & 0xff800000u) != hi || ex == 0u || n2 < lo || n3 < lo)
+    return;
+  const int32_t q = n3 - n2;
+  if (q == 0) { /* the increment rounds away: w is a fixed point */
+    *k = 0;
+    return;
+  }
+  const int32_t room = q > 0 ? fold_room(top - n3, q) : fold_room(n3 - lo, -q);
+  const int32_t j = room < *k ? room : *k;
+  *w = fold_float(hi | ((uint32_t)(n3 + j * q) & 0x007fffffu));
+  *k -= j;
+}
+
+/* w[e] after k sequential additions of d[e], for three folds of the same
+ * length (k > FOLD_SERIAL_MAX): their rounds interleave, because each one
+ * alone is a chain of dependent operations. */
+MOPCUDA_HD_SLOW void fold3_add_long(float w[3], const float d[3], int k) {
+  float v0 = w[0], v1 = w[1], v2 = w[2];
+  int k0 = k, k1 = k, k2 = k;
+  /* d = +-0, inf or NaN: after one addition the value is a fixed point */
+#define FOLD3_START(v, d, kk)                                                     \
+  if ((fold_bits(d) & 0x7fffffffu) == 0u || (fold_bits(d) & 0x7f800000u) == 0x7f800000u) { \
+    v = fold_fadd(v, d);                                                          \
+    kk = 0;                                                                       \
+  } else if ((fold_bits(v) & 0x7f800000u) == 0x7f800000u)                         \
+    kk = 0
+  FOLD3_START(v0, d[0], k0);
+  FOLD3_START(v1, d[1], k1);
+  FOLD3_START(v2, d[2], k2);
+#undef FOLD3_START
+  while ((k0 | k1 | k2) != 0) {
+    if (k0)
+      fold_round(&v0, d[0], &k0);
+    if (k1)
+      fold_round(&v1, d[1], &k1);
+    if (k2)
+      fold_round(&v2, d[2], &k2);
+  }
+  w[0] = v0;
+  w[1] = v1;
+  w[2] = v2;
 }
 
 /* w after k >= 0 sequential additions of d. */

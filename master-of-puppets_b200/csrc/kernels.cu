@@ -753,7 +753,7 @@ __device__ __forceinline__ bool rec_ordered(const FrameArgs &a, const RasterRec 
 }
 
 /* Records above the small-record limits (bbox side / area, tunable) are
- * rasterised item-parallel by k_raster_large. */
+ * rasterised by k_raster_large. */
 __device__ __forceinline__ bool rec_large(const FrameArgs &a, const RasterRec &r) {
   int w = (int)r.x1 - (int)r.x0 + 1, h = (int)(r.y1 & 0x7fffu) - (int)r.y0 + 1;
   return w > a.small_side || h > a.small_side || w * h > a.small_area;
@@ -765,21 +765,57 @@ __device__ __forceinline__ uint32_t rec_items(const RasterRec &r) {
   return h * ((w + RASTER_CHUNK - 1u) / RASTER_CHUNK);
 }
 
-/* Queue a large record for item-parallel rasterisation. */
+__device__ __forceinline__ uint32_t rec_chunks(const RasterRec &r) {
+  return ((uint32_t)r.x1 - (uint32_t)r.x0) / RASTER_CHUNK + 1u;
+}
+
 /* Queues a large record: one 64-bit atomic takes its list slot (high word)
  * and the offset of its first item (low word) together, so the offsets come
- * out ascending with the slot and no scan pass is needed.  An item total
- * past 2^32 carries into the slot count: flagged (bit 9), the frame fails. */
+ * out ascending with the slot and no scan pass is needed.  (An atomic per
+ * record: the setup of 20 views with many large records took 155 us, with the
+ * table's counter 290; with the group's shared ones 90.)  An item total
+ * past 2^32 carries into the slot count: flagged (bit 9), the frame fails.
+ * Its chunk_w entries are taken too; past the capacity it has none. */
 __device__ __forceinline__ void push_large(const FrameArgs &a, uint32_t rid, const RasterRec &r) {
-  const uint32_t n = rec_items(r);
-  const unsigned long long old = atomicAdd(
-      reinterpret_cast<unsigned long long *>(&a.ctr->large_items), (1ull << 32) | n);
-  const uint32_t q = (uint32_t)(old >> 32), off = (uint32_t)old;
-  if (off + n < off)
+  const uint32_t h = (uint32_t)(r.y1 & 0x7fffu) - (uint32_t)r.y0 + 1u, chunks = rec_chunks(r);
+  const bool wide = chunks > WIDE_CHUNKS;
+  const uint32_t n = wide ? (h + BAND_ROWS - 1u) / BAND_ROWS *
+                                ((chunks + BAND_CHUNKS - 1u) / BAND_CHUNKS)
+                          : h;
+  /* the converged lanes with the same list share the atomics: one lane adds
+   * the group's total and each takes its place behind the lanes below it */
+  const uint32_t mask = __activemask(), lane = threadIdx.x & 31u;
+  const uint32_t peers =
+      __match_any_sync(mask, (unsigned long long)(uintptr_t)a.ctr + (wide ? 1u : 0u));
+  uint32_t before_n = 0, sum_n = 0, before_e = 0, sum_e = 0;
+  for (uint32_t m = peers; m; m &= m - 1u) {
+    const uint32_t src = (uint32_t)__ffs((int)m) - 1u;
+    const uint32_t vn = __shfl_sync(peers, n, (int)src);
+    const uint32_t ve = __shfl_sync(peers, h * chunks, (int)src);
+    before_n += src < lane ? vn : 0u;
+    before_e += src < lane ? ve : 0u;
+    sum_n += vn;
+    sum_e += ve;
+  }
+  const int leader = __ffs((int)peers) - 1;
+  unsigned long long old = 0, e = 0;
+  if ((int)lane == leader) {
+    old = atomicAdd(reinterpret_cast<unsigned long long *>(wide ? &a.ctr->wide_items
+                                                                : &a.ctr->large_items),
+                    ((unsigned long long)__popc(peers) << 32) | sum_n);
+    e = atomicAdd(&a.ctr->chunk_count, (unsigned long long)sum_e);
+  }
+  old = __shfl_sync(peers, old, leader);
+  e = __shfl_sync(peers, e, leader);
+  const uint32_t q = (uint32_t)(old >> 32) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  const uint32_t off = (uint32_t)old + before_n;
+  if ((uint32_t)old + sum_n < sum_n)
     atomicOr(&a.ctr->overflow, 512u);
+  e += before_e;
+  a.large_off[rid] = e + h * chunks <= a.chunk_cap ? (uint32_t)e : 0xffffffffu;
   if (q < a.large_cap) {
-    a.large_list[q] = rid;
-    a.large_items[q] = off;
+    (wide ? a.wide_list : a.large_list)[q] = rid;
+    (wide ? a.wide_items : a.large_items)[q] = off;
   } else {
     atomicOr(&a.ctr->overflow, 8u);
   }
@@ -998,64 +1034,88 @@ __global__ void k_clip(FrameArgs a) {
  * exact tie the earliest submitted (strict `z < depth`, rasterizer.c:1960).
  * ------------------------------------------------------------------------ */
 /* Walk samples [xs, xe] of row y of record r, starting from edge values
- * w0..w2 (and flat depth z) already folded to (y, xs). */
-__device__ __forceinline__ void raster_span(const FrameArgs &a, const RasterRec &r, bool flat, int y,
-                                            int xs, int xe, float w0, float w1, float w2, float z) {
-  unsigned long long *row = a.keys + (size_t)y * (size_t)a.width;
-  bool seen = false;
-  for (int x = xs; x <= xe; x++) {
-    if (w0 >= 0.0f && w1 >= 0.0f && w2 >= 0.0f) {
-      seen = true;
+ * w0..w2 (and flat depth z) already folded to (y, xs); the whole warp calls it,
+ * `live` lanes have a row.  The edge values are monotone along a row, so its
+ * covered samples are consecutive: one loop steps to the first, a second one
+ * rasterises up to the last, and the warp meets between them.  (In one loop,
+ * lanes still before their coverage sit through the others' depth and atomic
+ * code: 131 us for 2 M triangles of 0.1-8 px at 1920x1080, and 45 us for
+ * 1.47 M at 3840x2160 samples, against 110 and 39; in two without the meeting
+ * point the lanes drift apart and run both loops a few at a time, 12 of 32
+ * active: 55 us for the latter.) */
+__device__ __forceinline__ void raster_span(const FrameArgs &a, const RasterRec &r, bool flat,
+                                            bool live, int y, int xs, int xe, float w0, float w1,
+                                            float w2, float z) {
+  int x = xs;
+  bool in = false;
+  if (live)
+    for (; x <= xe; x++) {
+      in = w0 >= 0.0f && w1 >= 0.0f && w2 >= 0.0f;
+      if (in)
+        break;
+      w0 = __fadd_rn(w0, r.dx[0]);
+      w1 = __fadd_rn(w1, r.dx[1]);
+      w2 = __fadd_rn(w2, r.dx[2]);
+      if (flat)
+        z = __fadd_rn(z, r.zc[1]);
+    }
+  __syncwarp();
+  if (in) {
+    unsigned long long *p = a.keys + (size_t)y * (size_t)a.width + x;
+    do {
       float zz = z;
       if (!flat) {
-        float b0 = w0 * r.inv_area, b1 = w1 * r.inv_area, b2 = w2 * r.inv_area;
+        const float b0 = w0 * r.inv_area, b1 = w1 * r.inv_area, b2 = w2 * r.inv_area;
         zz = b0 * r.zc[0] + b1 * r.zc[1] + b2 * r.zc[2];
       }
       if (zz < 1.0f)
-        atomicMin(row + x, ((unsigned long long)depth_key(zz) << 32) | (unsigned long long)r.order);
-    } else if (seen) {
-      break; /* edge values are monotone along a row: coverage has ended */
-    }
-    w0 = __fadd_rn(w0, r.dx[0]);
-    w1 = __fadd_rn(w1, r.dx[1]);
-    w2 = __fadd_rn(w2, r.dx[2]);
-    if (flat)
-      z = __fadd_rn(z, r.zc[1]);
+        atomicMin(p, ((unsigned long long)depth_key(zz) << 32) | (unsigned long long)r.order);
+      w0 = __fadd_rn(w0, r.dx[0]);
+      w1 = __fadd_rn(w1, r.dx[1]);
+      w2 = __fadd_rn(w2, r.dx[2]);
+      if (flat)
+        z = __fadd_rn(z, r.zc[1]);
+      x++;
+      p++;
+    } while (x <= xe && w0 >= 0.0f && w1 >= 0.0f && w2 >= 0.0f);
   }
+  __syncwarp();
 }
 
-/* Small records: one thread walks the whole (<= 128-sample) bbox, row by
- * row, exactly as the reference's loops step (rasterizer.c:1926-2151). */
+/* Small records: one thread walks the whole bbox, row by row, exactly as the
+ * reference's loops step (rasterizer.c:1926-2151), the warp's rows together. */
 __device__ __forceinline__ uint32_t raster_small_items(const FrameArgs &a) {
   const uint32_t n = a.total_tris + a.ctr->rec_count;
   return n > a.rec_cap ? a.rec_cap : n;
 }
 
-__device__ __forceinline__ void raster_small_item(const FrameArgs &a, uint32_t rid) {
-  {
-    const RasterRec r = a.rrec[rid];
-    if (!rec_live(r, a.width, a.height) || rec_large(a, r) || rec_ordered(a, r))
-      return;
-    const bool flat = (r.y1 & REC_FLAT_BIT) != 0;
-    const int y1 = (int)(r.y1 & 0x7fffu);
-    float wr0 = r.w0[0], wr1 = r.w0[1], wr2 = r.w0[2], zr = r.zc[0];
-    for (int y = (int)r.y0; y <= y1; y++) {
-      raster_span(a, r, flat, y, (int)r.x0, (int)r.x1, wr0, wr1, wr2, zr);
-      wr0 = __fadd_rn(wr0, r.dy[0]);
-      wr1 = __fadd_rn(wr1, r.dy[1]);
-      wr2 = __fadd_rn(wr2, r.dy[2]);
-      if (flat)
-        zr = __fadd_rn(zr, r.zc[2]);
-    }
+/* The whole warp calls it; `live` lanes have a record. */
+__device__ __forceinline__ void raster_small_item(const FrameArgs &a, bool live, uint32_t rid) {
+  RasterRec r;
+  if (live) {
+    r = a.rrec[rid];
+    live = rec_live(r, a.width, a.height) && !rec_large(a, r) && !rec_ordered(a, r);
+  }
+  const int rows = live ? (int)(r.y1 & 0x7fffu) - (int)r.y0 + 1 : 0;
+  const int n = (int)__reduce_max_sync(0xffffffffu, (unsigned)rows);
+  const bool flat = (r.y1 & REC_FLAT_BIT) != 0;
+  float wr0 = r.w0[0], wr1 = r.w0[1], wr2 = r.w0[2], zr = r.zc[0];
+  for (int j = 0; j < n; j++) {
+    raster_span(a, r, flat, j < rows, (int)r.y0 + j, (int)r.x0, (int)r.x1, wr0, wr1, wr2, zr);
+    wr0 = __fadd_rn(wr0, r.dy[0]);
+    wr1 = __fadd_rn(wr1, r.dy[1]);
+    wr2 = __fadd_rn(wr2, r.dy[2]);
+    if (flat)
+      zr = __fadd_rn(zr, r.zc[2]);
   }
 }
 
 __global__ void k_raster_small(FrameArgs a) {
   pdl_wait();
-  const uint32_t n = raster_small_items(a);
-  for (uint32_t rid = blockIdx.x * blockDim.x + threadIdx.x; rid < n;
-       rid += gridDim.x * blockDim.x)
-    raster_small_item(a, rid);
+  const uint32_t n = raster_small_items(a), lane = threadIdx.x & 31u;
+  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < n;
+       base += gridDim.x * blockDim.x)
+    raster_small_item(a, base + lane < n, base + lane);
 }
 
 /* Exclusive scan of a record list's item counts (the ordered, wireframe and
@@ -1122,50 +1182,278 @@ __device__ __forceinline__ void items_scan_block(T *items, uint32_t n, T *total_
     *total_out = carry;
 }
 
-/* Large records: one thread per (row, RASTER_CHUNK-sample chunk); the edge
- * values at the chunk start come from the exact fold. */
-__device__ __forceinline__ void raster_large_item(const FrameArgs &a, uint32_t it) {
-  uint32_t nl = a.ctr->large_count;
-  if (nl > a.large_cap)
-    nl = a.large_cap;
-  {
-    uint32_t lo = 0, hi = nl; /* last record with offset <= it */
-    while (hi - lo > 1) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (a.large_items[mid] <= it)
-        lo = mid;
-      else
-        hi = mid;
+/* The three edge values after k sequential additions of their increments
+ * (fold_add for each edge).  Folds up to FOLD3_SERIAL_MAX step the first two
+ * edges as one paired add (__fadd2_rn: two IEEE round-to-nearest single
+ * additions in one instruction) and the third alone, for as many steps as the
+ * longest such fold among the warp's converged lanes, each lane's steps past
+ * its own k predicated off; longer folds skip binades, the three edges'
+ * rounds interleaved.  A step is about 3 instructions and a round of the
+ * skipping fold about 120, of which a fold takes 5 to 20: with the line at
+ * 16 instead of 64, the rows of 20 views' large records took 497 instead of
+ * 364 us and their shading 1,580 instead of 1,314. */
+#define FOLD3_SERIAL_MAX 64
+__device__ __forceinline__ void fold3(float w[3], const float d[3], int k) {
+  if (k <= FOLD3_SERIAL_MAX) {
+    const int km = (int)__reduce_max_sync(__activemask(), (unsigned)k);
+    float2 p = make_float2(w[0], w[1]);
+    const float2 dp = make_float2(d[0], d[1]);
+    float q = w[2];
+#pragma unroll
+    for (int i = 0; i < FOLD_SERIAL_MAX; i++) {
+      if (i >= km)
+        break;
+      if (i < k) {
+        p = __fadd2_rn(p, dp);
+        q = __fadd_rn(q, d[2]);
+      }
     }
-    const uint32_t rid = a.large_list[lo];
-    if (rid >= a.rec_cap)
-      return;
-    const RasterRec r = a.rrec[rid];
-    if (!rec_live(r, a.width, a.height) || rec_ordered(a, r))
-      return;
-    const bool flat = (r.y1 & REC_FLAT_BIT) != 0;
-    const uint32_t w = (uint32_t)r.x1 - (uint32_t)r.x0 + 1u;
-    const uint32_t chunks = (w + RASTER_CHUNK - 1u) / RASTER_CHUNK;
-    const uint32_t local = it - a.large_items[lo];
-    const int jr = (int)(local / chunks), kc = (int)((local % chunks) * RASTER_CHUNK);
-    const int y = (int)r.y0 + jr;
-    if (y > (int)(r.y1 & 0x7fffu))
-      return;
-    const int xs = (int)r.x0 + kc, xe = min((int)r.x1, xs + RASTER_CHUNK - 1);
-    float w0 = fold_add(fold_add(r.w0[0], r.dy[0], jr), r.dx[0], kc);
-    float w1 = fold_add(fold_add(r.w0[1], r.dy[1], jr), r.dx[1], kc);
-    float w2 = fold_add(fold_add(r.w0[2], r.dy[2], jr), r.dx[2], kc);
-    float z = flat ? fold_add(fold_add(r.zc[0], r.zc[2], jr), r.zc[1], kc) : 0.0f;
-    raster_span(a, r, flat, y, xs, xe, w0, w1, w2, z);
+    for (int i = FOLD_SERIAL_MAX; i < km; i += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (i + u < k) {
+          p = __fadd2_rn(p, dp);
+          q = __fadd_rn(q, d[2]);
+        }
+    }
+    w[0] = p.x;
+    w[1] = p.y;
+    w[2] = q;
+  } else {
+    fold3_add_long(w, d, k);
   }
 }
 
-__global__ void k_raster_large(FrameArgs a) {
+/* ------------------------------------------------------------------------
+ * Large records, a warp at a time: 32 rows of narrow ones (at most
+ * WIDE_CHUNKS chunks wide), or a band of BAND_ROWS x BAND_CHUNKS chunks of a
+ * wide one.  Every
+ * chunk's edge values at its first sample are exact folds; they stay in
+ * chunk_w, so that shading one of its samples folds at most 31 steps instead
+ * of again from the record's corner (64 views' shading 3.83 -> 2.97 ms).  Chunks with a sample that may be
+ * covered go through a queue in shared memory and are walked 32 at a time,
+ * a lane each, so that empty ones (about half of a wide triangle's box) take
+ * no lane.
+ * As independent (row, chunk) items of a thread each, every chunk folded
+ * both ways from the corner and searched its record alone: a ground plane of
+ * two triangles took 21 us at 800x600 (now 17) and 102 us at 2403x1347 (now
+ * 47), 20 views' large records 530 us (now 376).
+ * ------------------------------------------------------------------------ */
+#define LARGE_WARPS 8
+struct LargeSmem {
+  float4 w[64]; /* queue: edge values (and flat depth) at a chunk's start */
+  uint32_t rid[64];
+  uint32_t xy[64]; /* y << 16 | x of its first sample */
+  float4 start[BAND_ROWS * BAND_CHUNKS];
+};
+
+/* List slot of the record that item `it` of a list (n > 0 entries) belongs to:
+ * the last one with offset <= it, found by the whole warp. */
+__device__ __forceinline__ uint32_t warp_slot(const uint32_t *items, uint32_t n, uint32_t it) {
+  uint32_t lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const uint32_t step = (hi - lo + 31u) >> 5;
+    const uint32_t cand = lo + (threadIdx.x & 31u) * step;
+    const uint32_t pass = __ballot_sync(0xffffffffu, cand < hi && items[cand] <= it);
+    lo += (uint32_t)(31 - __clz((int)pass)) * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
+/* True when no sample of the chunk (n + 1 samples from edge values w) is
+ * covered: some edge value is negative at its largest end.  The values along
+ * a row are monotone (each step adds the same increment and rounding is
+ * monotone), so the first value is the largest where the increment is not
+ * positive; where it is positive, the last one is bounded by the sum without
+ * rounding plus the roundings' bound (each at most 2^-24 of the largest
+ * magnitude, fewer than 32 of them; taken twice). */
+__device__ __forceinline__ bool chunk_empty(const float4 &w, const RasterRec &r, int n) {
+  const float v[3] = {w.x, w.y, w.z};
+  bool empty = false;
+#pragma unroll
+  for (int e = 0; e < 3; e++) {
+    const float end = v[e] + (float)n * r.dx[e];
+    const float err = fmaxf(fabsf(v[e]), fabsf(end)) * (64.0f / 16777216.0f);
+    empty |= v[e] < 0.0f && (!(r.dx[e] > 0.0f) || end + err < 0.0f);
+  }
+  return empty;
+}
+
+/* Walks the queue's entries [first, first + n), n <= 32, a lane each. */
+__device__ __forceinline__ void large_walk(const FrameArgs &a, const LargeSmem &q, uint32_t first,
+                                           uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  RasterRec r;
+  float4 w;
+  int x = 0, y = 0;
+  if (lane < n) {
+    const uint32_t k = first + lane;
+    r = a.rrec[q.rid[k]];
+    w = q.w[k];
+    x = (int)(q.xy[k] & 0xffffu);
+    y = (int)(q.xy[k] >> 16);
+  }
+  raster_span(a, r, (r.y1 & REC_FLAT_BIT) != 0, lane < n, y, x,
+              min((int)r.x1, x + RASTER_CHUNK - 1), w.x, w.y, w.z, w.w);
+}
+
+/* Adds the chunk of each lane with `live` to the queue of n entries (fewer
+ * than 32) and walks 32 of them when there are that many. */
+__device__ __forceinline__ void large_push(const FrameArgs &a, LargeSmem &q, uint32_t &n, bool live,
+                                           uint32_t rid, int x, int y, const float4 &w) {
+  const uint32_t m = __ballot_sync(0xffffffffu, live);
+  if (live) {
+    const uint32_t k = n + (uint32_t)__popc(m & ((1u << (threadIdx.x & 31u)) - 1u));
+    q.w[k] = w;
+    q.rid[k] = rid;
+    q.xy[k] = ((uint32_t)y << 16) | (uint32_t)x;
+  }
+  n += (uint32_t)__popc(m);
+  __syncwarp();
+  if (n >= 32u) {
+    n -= 32u;
+    large_walk(a, q, n, 32u);
+  }
+}
+
+/* Rows [base, base + 32) of the narrow list (base warp-uniform). */
+__device__ __forceinline__ void narrow_rows(const FrameArgs &a, uint32_t base, LargeSmem &q,
+                                            uint32_t &n) {
+  const uint32_t it = base + (threadIdx.x & 31u), total = a.ctr->large_items;
+  const uint32_t nl = min(a.ctr->large_count, a.large_cap);
+  /* one search for the first row's record, then each lane's own among the
+   * records that 32 consecutive rows can touch */
+  uint32_t lo = warp_slot(a.large_items, nl, base), hi = min(nl, lo + 33u);
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (a.large_items[mid] <= it)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  const uint32_t rid = a.large_list[lo], jr = it - a.large_items[lo];
+  bool live = it < total && rid < a.rec_cap;
+  RasterRec r;
+  if (live) {
+    r = a.rrec[rid];
+    live = rec_live(r, a.width, a.height) && !rec_ordered(a, r) &&
+           (int)r.y0 + (int)jr <= (int)(r.y1 & 0x7fffu);
+  }
+  const bool flat = (r.y1 & REC_FLAT_BIT) != 0;
+  float e[3] = {r.w0[0], r.w0[1], r.w0[2]};
+  float z = 0.0f;
+  uint32_t ci = 0xffffffffu;
+  if (live) {
+    fold3(e, r.dy, (int)jr);
+    if (flat)
+      z = fold_add(r.zc[0], r.zc[2], (int)jr);
+    ci = a.large_off[rid];
+  }
+  const uint32_t chunks = live ? rec_chunks(r) : 0u;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, chunks);
+  for (uint32_t c = 0;;) {
+    const float4 w = make_float4(e[0], e[1], e[2], z);
+    const int x = (int)r.x0 + (int)c * RASTER_CHUNK;
+    live = c < chunks;
+    if (live && ci != 0xffffffffu)
+      a.chunk_w[ci + jr * chunks + c] = w;
+    live = live && !chunk_empty(w, r, min((int)r.x1 - x, RASTER_CHUNK - 1));
+    large_push(a, q, n, live, rid, x, (int)r.y0 + (int)jr, w);
+    if (++c >= most)
+      break;
+    if (c < chunks) { /* to the next chunk, step by step */
+#pragma unroll 8
+      for (int k = 0; k < RASTER_CHUNK; k++) {
+        for (int s = 0; s < 3; s++)
+          e[s] = __fadd_rn(e[s], r.dx[s]);
+        if (flat)
+          z = __fadd_rn(z, r.zc[1]);
+      }
+    }
+  }
+}
+
+/* Band `it` of the wide list.  Lane (row, value) folds one of the row's three
+ * edge values (or its flat depth) to the row, then to the band's first column,
+ * and steps along the band as the reference does, leaving the value at every
+ * chunk's start: the long folds run once per row and band. */
+__device__ __forceinline__ void wide_band(const FrameArgs &a, uint32_t it, LargeSmem &q,
+                                          uint32_t &n) {
+  static_assert(BAND_ROWS == 8 && BAND_CHUNKS == 8, "a lane per row and value, two chunks per lane");
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t slot = warp_slot(a.wide_items, min(a.ctr->wide_count, a.large_cap), it);
+  const uint32_t rid = a.wide_list[slot];
+  if (rid >= a.rec_cap)
+    return;
+  const RasterRec r = a.rrec[rid];
+  if (!rec_live(r, a.width, a.height) || rec_ordered(a, r))
+    return;
+  const int h = (int)(r.y1 & 0x7fffu) - (int)r.y0 + 1, chunks = (int)rec_chunks(r);
+  const uint32_t cols = ((uint32_t)chunks + BAND_CHUNKS - 1u) / BAND_CHUNKS;
+  const uint32_t band = it - a.wide_items[slot];
+  const int j0 = (int)(band / cols) * BAND_ROWS, c0 = (int)(band % cols) * BAND_CHUNKS;
+  if (j0 >= h)
+    return;
+  {
+    const uint32_t c = lane & 3u;
+    const bool used = c < 3u || (r.y1 & REC_FLAT_BIT) != 0;
+    float v = c == 0u ? r.w0[0] : c == 1u ? r.w0[1] : c == 2u ? r.w0[2] : r.zc[0];
+    float dy = c == 0u ? r.dy[0] : c == 1u ? r.dy[1] : c == 2u ? r.dy[2] : r.zc[2];
+    float dx = c == 0u ? r.dx[0] : c == 1u ? r.dx[1] : c == 2u ? r.dx[2] : r.zc[1];
+    if (!used)
+      v = dy = dx = 0.0f;
+    v = fold_add(fold_add(v, dy, j0 + (int)(lane >> 2)), dx, c0 * RASTER_CHUNK);
+    float *st = reinterpret_cast<float *>(&q.start[(lane >> 2) * BAND_CHUNKS]) + c;
+    const int nc = min(BAND_CHUNKS, chunks - c0);
+    for (int k = 0; k < nc; k++) {
+      st[4 * k] = v;
+#pragma unroll
+      for (int s = 0; s < RASTER_CHUNK; s++)
+        v = __fadd_rn(v, dx);
+    }
+  }
+  __syncwarp();
+  const uint32_t ci = a.large_off[rid];
+#pragma unroll
+  for (uint32_t i = lane; i < BAND_ROWS * BAND_CHUNKS; i += 32u) {
+    const int j = j0 + (int)(i / BAND_CHUNKS), c = c0 + (int)(i % BAND_CHUNKS);
+    const int x = (int)r.x0 + c * RASTER_CHUNK;
+    bool live = j < h && c < chunks;
+    const float4 w = q.start[i];
+    if (live && ci != 0xffffffffu)
+      a.chunk_w[ci + (uint32_t)(j * chunks + c)] = w;
+    live = live && !chunk_empty(w, r, min((int)r.x1 - x, RASTER_CHUNK - 1));
+    large_push(a, q, n, live, rid, x, (int)r.y0 + j, w);
+  }
+  __syncwarp(); /* start is read before the next band replaces it */
+}
+
+/* Work of the warps: the bands, then the rows 32 at a time. */
+__device__ __forceinline__ uint32_t large_units(const FrameArgs &a) {
+  const uint32_t rows = a.ctr->large_items;
+  return a.ctr->wide_items + rows / 32u + (rows % 32u ? 1u : 0u);
+}
+
+__device__ __forceinline__ void large_unit(const FrameArgs &a, uint32_t u, LargeSmem &q,
+                                           uint32_t &n) {
+  const uint32_t bands = a.ctr->wide_items;
+  if (u < bands)
+    wide_band(a, u, q, n);
+  else
+    narrow_rows(a, (u - bands) * 32u, q, n);
+}
+
+__global__ void __launch_bounds__(32 * LARGE_WARPS) k_raster_large(FrameArgs a) {
   pdl_wait();
-  const uint32_t total = a.ctr->large_items;
-  for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < total;
-       it += gridDim.x * blockDim.x)
-    raster_large_item(a, it);
+  __shared__ LargeSmem sq[LARGE_WARPS];
+  LargeSmem &q = sq[threadIdx.x >> 5];
+  const uint32_t units = large_units(a);
+  uint32_t n = 0;
+  for (uint32_t u = blockIdx.x * LARGE_WARPS + (threadIdx.x >> 5); u < units;
+       u += gridDim.x * LARGE_WARPS)
+    large_unit(a, u, q, n);
+  large_walk(a, q, 0u, n);
 }
 
 /* ------------------------------------------------------------------------
@@ -1361,37 +1649,6 @@ __global__ void __launch_bounds__(256) k_resolve(FrameArgs a) {
   }
 }
 
-/* The three edge values after k sequential additions of their increments
- * (fold_add for each edge).  Short folds (k <= FOLD_SERIAL_MAX) step the
- * first two edges as one paired add (__fadd2_rn: two IEEE round-to-nearest
- * single additions in one instruction) and the third alone, for as many
- * steps as the longest short fold among the warp's converged lanes, each
- * lane's steps past its own k predicated off; longer folds take the
- * binade-skipping path per edge. */
-__device__ __forceinline__ void fold3(float w[3], const float d[3], int k) {
-  if (k <= FOLD_SERIAL_MAX) {
-    const int km = (int)__reduce_max_sync(__activemask(), (unsigned)k);
-    float2 p = make_float2(w[0], w[1]);
-    const float2 dp = make_float2(d[0], d[1]);
-    float q = w[2];
-#pragma unroll
-    for (int i = 0; i < FOLD_SERIAL_MAX; i++) {
-      if (i >= km)
-        break;
-      if (i < k) {
-        p = __fadd2_rn(p, dp);
-        q = __fadd_rn(q, d[2]);
-      }
-    }
-    w[0] = p.x;
-    w[1] = p.y;
-    w[2] = q;
-  } else {
-    for (int e = 0; e < 3; e++)
-      w[e] = fold_add_long(w[e], d[e], k);
-  }
-}
-
 /* Edge values of record r at row jr, column kc of its bbox: the row fold
  * from the corner, then the column fold along the row, as the reference
  * steps them. */
@@ -1455,7 +1712,22 @@ __device__ __forceinline__ void shade_item(const FrameArgs &a, uint32_t j, const
     const ShadeRec s = a.srec[rid];
     const DrawRec &d = a.draws[s.draw < a.draw_count ? s.draw : 0];
     const LightRec *Ls = lights + d.light_off;
-    const int jr = y - (int)r.y0, kc = x - (int)r.x0;
+    int jr = y - (int)r.y0, kc = x - (int)r.x0;
+    /* a large record's sample folds from its chunk's stored values, as if the
+     * box began there */
+    if (rec_large(a, r)) {
+      const uint32_t ci = a.large_off[rid];
+      if (ci != 0xffffffffu) {
+        const float4 cw = a.chunk_w[ci + (uint32_t)jr * rec_chunks(r) + (uint32_t)kc / RASTER_CHUNK];
+        r.w0[0] = cw.x;
+        r.w0[1] = cw.y;
+        r.w0[2] = cw.z;
+        if (r.y1 & REC_FLAT_BIT)
+          r.zc[0] = cw.w;
+        jr = 0;
+        kc %= RASTER_CHUNK;
+      }
+    }
     float hdr[3], depth;
     if (r.y1 & REC_FLAT_BIT) {
       depth = fold_add(fold_add(r.zc[0], r.zc[2], jr), r.zc[1], kc);
@@ -3203,6 +3475,8 @@ __global__ void __launch_bounds__(256) k_batch_prepare(BatchArgs b) {
     a.height = vw.height;
     a.keys = b.keys + vw.sample_off;
     a.shade_list = b.shade_list + vw.sample_off;
+    a.chunk_w = b.chunk_w + vw.sample_off / 2ull;
+    a.chunk_cap = chunk_entries((unsigned long long)vw.width * (unsigned long long)vw.height);
     a.pre = b.pre + vw.sample_off;
     a.depth = b.depth + vw.sample_off;
     a.ids = b.ids + vw.sample_off;
@@ -3324,11 +3598,14 @@ __global__ void __launch_bounds__(256) k_batch_alloc(BatchArgs b) {
       a.vertex_cap = (uint32_t)need[0];
       a.rrec = b.rrec + off[1];
       a.srec = b.srec + off[1];
+      a.large_off = b.large_off + off[1];
       a.rec_cap = (uint32_t)need[1];
       a.clipq = b.clipq + off[2];
       a.clip_cap = (uint32_t)need[2];
       a.large_list = b.large_list + off[3];
       a.large_items = b.large_items + off[3];
+      a.wide_list = b.wide_list + off[3];
+      a.wide_items = b.wide_items + off[3];
       a.large_cap = (uint32_t)need[3];
       if (a.hdr) {
         a.olist = b.olist + off[4];
@@ -3368,10 +3645,10 @@ template <int ST> __device__ __forceinline__ uint32_t stage_count(const FrameArg
     return a.total_tris;
   case ST_CLIP:
     return clip_items(a);
-  case ST_RSMALL:
-    return a.total_tris ? raster_small_items(a) : 0u;
+  case ST_RSMALL: /* groups of 32 records */
+    return a.total_tris ? (raster_small_items(a) + 31u) / 32u : 0u;
   case ST_RLARGE:
-    return a.total_tris ? a.ctr->large_items : 0u;
+    return a.total_tris ? large_units(a) : 0u;
   case ST_SHADE:
     return a.ctr->shade_count;
   case ST_OCOUNT:
@@ -3434,13 +3711,47 @@ __global__ void __launch_bounds__(256) k_b_items(const FrameArgs *__restrict__ f
       vertex_item(a, i);
     else if (ST == ST_SETUP)
       setup_item<SH>(a, i);
-    else if (ST == ST_CLIP)
-      clip_item<SH>(a, i);
-    else if (ST == ST_RSMALL)
-      raster_small_item(a, i);
     else
-      raster_large_item(a, i);
+      clip_item<SH>(a, i);
   }
+}
+
+/* k_raster_small over every viewport's records: 32 at a time from one. */
+__global__ void __launch_bounds__(256) k_b_rsmall(const FrameArgs *__restrict__ fr, uint32_t nv) {
+  __shared__ uint32_t s_pre[MOPCUDA_MAX_VIEWS + 1];
+  const uint32_t total = views_prefix<ST_RSMALL>(fr, nv, s_pre), lane = threadIdx.x & 31u;
+  uint32_t v = 0;
+  for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < total;
+       g += (gridDim.x * blockDim.x) >> 5) {
+    while (s_pre[v + 1] <= g)
+      v++;
+    const FrameArgs &a = fr[v];
+    const uint32_t i = (g - s_pre[v]) * 32u + lane;
+    raster_small_item(a, i < raster_small_items(a), i);
+  }
+}
+
+/* k_raster_large over every viewport's units. */
+__global__ void __launch_bounds__(32 * LARGE_WARPS) k_b_rlarge(const FrameArgs *__restrict__ fr,
+                                                              uint32_t nv) {
+  __shared__ uint32_t s_pre[MOPCUDA_MAX_VIEWS + 1];
+  __shared__ LargeSmem sq[LARGE_WARPS];
+  const uint32_t total = views_prefix<ST_RLARGE>(fr, nv, s_pre);
+  LargeSmem &q = sq[threadIdx.x >> 5];
+  uint32_t v = 0, n = 0;
+  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < total;
+       u += (gridDim.x * blockDim.x) >> 5) {
+    uint32_t vu = v;
+    while (s_pre[vu + 1] <= u)
+      vu++;
+    if (vu != v) { /* the queue holds one viewport's chunks */
+      large_walk(fr[v], q, 0u, n);
+      n = 0;
+      v = vu;
+    }
+    large_unit(fr[v], u - s_pre[v], q, n);
+  }
+  large_walk(fr[v], q, 0u, n);
 }
 
 __global__ void __launch_bounds__(256) k_b_resolve(const FrameArgs *__restrict__ fr,
@@ -3638,8 +3949,8 @@ void mopcuda_batch_grids(BatchLaunch &cfg) {
   cfg.grid_vertex = grid((const void *)k_b_items<ST_VERTEX, false>, cfg.vertex_block);
   cfg.grid_setup = grid((const void *)k_b_items<ST_SETUP, false>, cfg.setup_block);
   cfg.grid_clip = grid((const void *)k_b_items<ST_CLIP, false>, 128);
-  cfg.grid_rsmall = grid((const void *)k_b_items<ST_RSMALL, false>, cfg.raster_block);
-  cfg.grid_rlarge = grid((const void *)k_b_items<ST_RLARGE, false>, cfg.large_block);
+  cfg.grid_rsmall = grid((const void *)k_b_rsmall, cfg.raster_block);
+  cfg.grid_rlarge = grid((const void *)k_b_rlarge, cfg.large_block);
   cfg.grid_shade = grid((const void *)k_b_shade<false>, cfg.shade_block);
 }
 
@@ -3666,8 +3977,8 @@ int mopcuda_launch_batch(const BatchArgs &b, const PostArgs *posts, const uint32
       k_b_items<ST_SETUP, false><<<cfg.grid_setup, cfg.setup_block, 0, s>>>(fr, nv);
       k_b_items<ST_CLIP, false><<<cfg.grid_clip, 128, 0, s>>>(fr, nv);
     }
-    k_b_items<ST_RSMALL, false><<<cfg.grid_rsmall, cfg.raster_block, 0, s>>>(fr, nv);
-    k_b_items<ST_RLARGE, false><<<cfg.grid_rlarge, cfg.large_block, 0, s>>>(fr, nv);
+    k_b_rsmall<<<cfg.grid_rsmall, cfg.raster_block, 0, s>>>(fr, nv);
+    k_b_rlarge<<<cfg.grid_rlarge, cfg.large_block, 0, s>>>(fr, nv);
     k_b_resolve<<<sms * 8, 256, 0, s>>>(fr, nv);
     if (shadows)
       k_b_shade<true><<<cfg.grid_shade, cfg.shade_block, 0, s>>>(fr, nv, shared_lights ? 1 : 0);

@@ -152,8 +152,8 @@ extern "C" void mopcuda_device_destroy(MopCudaDevice *d) {
   DevArena *arenas[] = {&d->irr,      &d->pf,         &d->brdf,        &d->d_draws,
                         &d->d_lights, &d->clip,       &d->world,       &d->normal,
                         &d->color,    &d->rrec,       &d->srec,
-                        &d->clipq,    &d->keys[0],    &d->keys[1],     &d->large_list,
-                        &d->large_items,
+                        &d->clipq,    &d->keys[0],    &d->keys[1],     &d->large_lists,
+                        &d->chunk_w,
                         &d->shade_list, &d->counters, &d->pick_xy,     &d->pick_out,
                         &d->deform_params, &d->hdr, &d->frag_head, &d->frags, &d->touched,
                         &d->olist, &d->olist_items, &d->wlist, &d->wlist_items, &d->wplots, &d->oscratch, &d->sh_map[0], &d->sh_map[1], &d->sh_d_draws,
@@ -1082,7 +1082,7 @@ static int launch_frame(MopCudaDevice *d) {
   rc |= d->normal.ensure(16ull * vcap);
   rc |= d->color.ensure(16ull * vcap);
   rc |= d->rrec.ensure(sizeof(RasterRec) * (size_t)rcap);
-  rc |= d->srec.ensure(sizeof(ShadeRec) * (size_t)rcap);
+  rc |= d->srec.ensure((sizeof(ShadeRec) + 4) * (size_t)rcap); /* and large_off */
   rc |= d->clipq.ensure(4ull * ccap);
   for (int i = 0; i < 2; i++) {
     const void *was = d->keys[i].p;
@@ -1090,8 +1090,8 @@ static int launch_frame(MopCudaDevice *d) {
     if (d->keys[i].p != was)
       d->keys_clean[i] = 0;
   }
-  rc |= d->large_list.ensure(4ull * lcap);
-  rc |= d->large_items.ensure(4ull * lcap);
+  rc |= d->large_lists.ensure(16ull * lcap);
+  rc |= d->chunk_w.ensure(16ull * chunk_entries(S));
   rc |= d->shade_list.ensure(4ull * S);
   rc |= d->counters.ensure(sizeof(Counters));
   rc |= d->h_draws.ensure(sizeof(DrawRec) * (nd ? nd : 1));
@@ -1159,9 +1159,14 @@ static int launch_frame(MopCudaDevice *d) {
   const int kb = d->keys_cur;
   a.keys = d->keys[kb].as<unsigned long long>();
   a.keys_next = d->keys[kb ^ 1].as<unsigned long long>();
-  a.large_list = d->large_list.as<uint32_t>();
-  a.large_items = d->large_items.as<uint32_t>();
+  a.large_list = d->large_lists.as<uint32_t>();
+  a.large_items = a.large_list + lcap;
+  a.wide_list = a.large_items + lcap;
+  a.wide_items = a.wide_list + lcap;
   a.large_cap = lcap;
+  a.large_off = (uint32_t *)(d->srec.as<ShadeRec>() + rcap);
+  a.chunk_w = d->chunk_w.as<float4>();
+  a.chunk_cap = chunk_entries(S);
   a.shade_list = d->shade_list.as<uint32_t>();
   a.ctr = d->counters.as<Counters>();
   memcpy(a.clear, d->clear, sizeof a.clear);
@@ -1324,7 +1329,8 @@ static int finish_frame(MopCudaDevice *d, int timeout_ms, bool defer_readback) {
     d->rec_hint = c->rec_count + c->rec_count / 4 + 1024;
     d->clip_hint = c->clip_count + c->clip_count / 4 + 1024;
     d->extra_hint = c->extra_vertices + c->extra_vertices / 4 + 1024;
-    d->large_hint = c->large_count + c->large_count / 4 + 1024;
+    const uint32_t large = std::max(c->large_count, c->wide_count);
+    d->large_hint = large + large / 4 + 1024;
     if (c->overflow & 16u)
       d->frag_hint = c->frag_count + c->frag_count / 4 + 65536;
     if (c->overflow & 32u)

@@ -142,11 +142,14 @@ struct __align__(16) ShadeRec {
 struct alignas(8) Counters {
   uint32_t rec_count;         /* fan records of clipped triangles (overflow region) */
   uint32_t extra_vertices;
-  /* one 64-bit counter: low word the items of the large records pushed so far
-   * (their list offsets, ascending with the list index), high word the number
-   * of large records (rasterised as (row, chunk) items); 8-byte aligned */
+  /* one 64-bit counter: low word the items (rows) of the narrow large records
+   * pushed so far (their list offsets, ascending with the list index), high
+   * word the number of these records; 8-byte aligned */
   uint32_t large_items;
   uint32_t large_count;
+  /* the same pair for the wide ones (their items: bands) */
+  uint32_t wide_items;
+  uint32_t wide_count;
   uint32_t clip_count;
   uint32_t overflow;          /* bit0 records, bit1 extra vertices, bit2 clip
                                  queue, bit3 large list, bit9 large-record
@@ -159,10 +162,13 @@ struct alignas(8) Counters {
   uint32_t scratch_count;          /* sort-scratch entries taken by long lists */
   uint32_t wlong_count;            /* samples of wireframe frames with a long list */
   uint32_t pad;
+  unsigned long long chunk_count;  /* chunk_w entries asked for by large records */
 };
 /* arrays of counters (one per viewport) keep the 64-bit pair aligned */
-static_assert(sizeof(Counters) % 8 == 0 && offsetof(Counters, large_items) % 8 == 0,
-              "large-record counter pair must be 8-byte aligned");
+static_assert(sizeof(Counters) % 8 == 0 && offsetof(Counters, large_items) % 8 == 0 &&
+                  offsetof(Counters, wide_items) % 8 == 0 &&
+                  offsetof(Counters, chunk_count) % 8 == 0,
+              "large-record counter pairs must be 8-byte aligned");
 
 /* Blended fragments of one sample sorted in registers; a sample with more
  * sorts its list in the fold's global scratch (heapsort). */
@@ -177,6 +183,19 @@ static_assert(sizeof(Counters) % 8 == 0 && offsetof(Counters, large_items) % 8 =
 #define SMALL_MAX_SIDE 32  /* default small-record limits */
 #define SMALL_MAX_AREA 128
 #define RASTER_CHUNK 32
+/* Large records wider than WIDE_CHUNKS chunks are rasterised in bands of
+ * BAND_ROWS rows by BAND_CHUNKS chunks, the others by rows. */
+#define WIDE_CHUNKS 4
+#define BAND_ROWS 8
+#define BAND_CHUNKS 8
+/* Chunk start entries a frame of `samples` samples keeps (16 B each); the
+ * shading folds the samples of records beyond them from the record's corner.
+ * Half the samples holds every row of a frame covered by boxes a dozen
+ * samples wide with some overlap; with a quarter, part of 64 views' records
+ * had none and their shading took 3.25 instead of 2.97 ms. */
+__host__ __device__ static inline uint32_t chunk_entries(unsigned long long samples) {
+  return (uint32_t)(samples / 2ull);
+}
 
 struct FrameArgs {
   const DrawRec *draws;
@@ -202,9 +221,15 @@ struct FrameArgs {
   unsigned long long *keys;         /* per sample: depth_key << 32 | order */
   unsigned long long *keys_next;    /* the next frame's key buffer, cleared by k_shade
                                        (null: none) */
-  uint32_t *large_list;             /* record ids of large records */
+  uint32_t *large_list;             /* record ids of narrow large records */
   uint32_t *large_items;            /* offset of each one's first item (ascending) */
-  uint32_t large_cap;
+  uint32_t *wide_list, *wide_items; /* the same of the wide ones */
+  uint32_t large_cap;               /* entries of either list */
+  uint32_t *large_off;              /* per record slot, large records only: its first chunk_w
+                                       entry (row by row, a row's chunks in order) */
+  float4 *chunk_w;                  /* the edge values (and the flat depth) at a chunk's first
+                                       sample, entries below chunk_cap */
+  uint32_t chunk_cap;
   uint32_t *shade_list;             /* covered sample indices */
   Counters *ctr;
   /* resolve */
@@ -362,10 +387,8 @@ __device__ __forceinline__ uint8_t x86_f2u8(float f) { return (uint8_t)(uint32_t
 /* Order-preserving map of a depth value to 32 bits; -0 and +0 share a key
  * (they compare equal under the reference's strict `<` test). */
 __device__ __forceinline__ uint32_t depth_key(float z) {
-  uint32_t b = __float_as_uint(z);
-  if ((b & 0x7fffffffu) == 0u)
-    b = 0u;
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  const uint32_t b = __float_as_uint(__fadd_rn(z, 0.0f)); /* -0 + 0 = +0 */
+  return b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
 }
 
 #define KEY_EMPTY 0xffffffffffffffffull
@@ -472,8 +495,10 @@ struct BatchArgs {
   unsigned long long rec_pool;
   uint32_t *clipq;
   unsigned long long clip_pool;
-  uint32_t *large_list, *large_items;
+  uint32_t *large_list, *large_items, *wide_list, *wide_items;
   unsigned long long large_pool;
+  uint32_t *large_off; /* rec_pool entries */
+  float4 *chunk_w;     /* chunk_entries(samples), at the viewports' sample offsets / 2 */
   unsigned long long *keys;
   uint32_t *shade_list;
   uchar4 *pre;
