@@ -161,7 +161,7 @@ struct alignas(8) Counters {
   uint32_t wire_count, wire_items; /* wireframe records queued, their plots */
   uint32_t scratch_count;          /* sort-scratch entries taken by long lists */
   uint32_t wlong_count;            /* samples of wireframe frames with a long list */
-  uint32_t pad;
+  uint32_t shade_next;             /* samples of the shading list handed out */
   unsigned long long chunk_count;  /* chunk_w entries asked for by large records */
 };
 /* arrays of counters (one per viewport) keep the 64-bit pair aligned */
@@ -471,6 +471,8 @@ struct BatchStatus {
                         record lists; bit8 a viewport with an ordered suffix or wireframe
                         draws in a launch without the buffers for them */
   uint32_t scratch_count; /* the fold's sort scratch, shared by the viewports */
+  uint32_t shade_next;    /* shading groups handed out */
+  uint32_t pad;
   unsigned long long need_vertex, need_rec, need_clip, need_large, need_olist, need_frag,
       need_wlist;
 };
