@@ -248,7 +248,7 @@ __device__ __forceinline__ float4 env_bilinear(const float4 *__restrict__ d, int
   float fx = u * (float)(w - 1);
   float fy = v * (float)(h - 1);
   int x0 = (int)fx, y0 = (int)fy;
-  int x1 = (x0 + 1) % w;
+  int x1 = x0 + 1 < w ? x0 + 1 : 0;
   int y1 = y0 + 1;
   if (y1 >= h)
     y1 = h - 1;

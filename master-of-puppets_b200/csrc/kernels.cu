@@ -277,8 +277,6 @@ __device__ float diffuse_flat(const FrameArgs &a, V3 n, V3 wp, const LightRec *L
   float total = amb;
   for (uint32_t i = 0; i < cnt; i++) {
     const LightRec &L = Ls[i];
-    if (!L.active)
-      continue;
     float ndotl = 0.0f, att = 1.0f, spot = 1.0f;
     if (L.type == 0) {
       V3 dir = mk3(L.ndir[0], L.ndir[1], L.ndir[2]);
@@ -313,6 +311,16 @@ __device__ float diffuse_flat(const FrameArgs &a, V3 n, V3 wp, const LightRec *L
   return clamp01(total);
 }
 
+__device__ __forceinline__ LightRec load_light(const LightRec *p) {
+  LightRec L;
+  float4 *d = reinterpret_cast<float4 *>(&L);
+  const float4 *s = reinterpret_cast<const float4 *>(p);
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    d[k] = s[k];
+  return L;
+}
+
 /* compute_multi_light_rgb (rasterizer.c:1596-1688) and
  * compute_multi_specular_ggx (1701-1814) evaluated in one pass over the
  * lights.  For point and spot lights both reference helpers compute the same
@@ -335,9 +343,7 @@ __device__ void lights_smooth(const FrameArgs &a, V3 n, V3 wp, V3 vdir, const Li
   const float g1v = ndotv / (ndotv * omk + k);
   const uint32_t cnt = d.light_count;
   for (uint32_t i = 0; i < cnt; i++) {
-    const LightRec &L = Ls[i];
-    if (!L.active)
-      continue;
+    const LightRec L = load_light(Ls + i);
     float ndl_d = 0.0f, ndl_s, att = 1.0f, spot = 1.0f;
     V3 ldir;
     if (L.type == 0) {
@@ -408,7 +414,7 @@ __device__ __forceinline__ void ibl_bilinear(const float *d, int w, int h, float
   int x0 = (int)fx, y0 = (int)fy;
   x0 = x0 < 0 ? 0 : (x0 > w - 1 ? w - 1 : x0);
   y0 = y0 < 0 ? 0 : (y0 > h - 1 ? h - 1 : y0);
-  int x1 = (x0 + 1) % w;
+  int x1 = x0 + 1 < w ? x0 + 1 : 0;
   int y1 = y0 + 1 < h ? y0 + 1 : h - 1;
   float sx = fx - (float)x0, sy = fy - (float)y0;
   const float4 p00 = __ldg((const float4 *)d + ((size_t)y0 * w + x0));
@@ -424,6 +430,18 @@ __device__ __forceinline__ void ibl_bilinear(const float *d, int w, int h, float
   }
 }
 
+/* x / c for a compile-time c, by Markstein's final step (P. Markstein, IBM J.
+ * Res. Dev. 34(1), 1990): q = x * RN(1/c) corrected by its exact remainder
+ * rounds correctly when neither underflows.  For the two divisors here the
+ * sum with 0.5 that follows equals the division's for every float x below
+ * 1e30 (checked exhaustively), tiny quotients being absorbed; 3 instructions
+ * instead of a division's dozen. */
+__device__ __forceinline__ float div_const(float x, float c) {
+  const float rc = 1.0f / c; /* folded by the compiler */
+  const float q = x * rc;
+  return __fmaf_rn(__fmaf_rn(-q, c, x), rc, q);
+}
+
 /* dir_to_uv, rasterizer.c:216-222.  atan2f/asinf are CUDA's; glibc's differ
  * in the last ulp for some inputs, which perturbs IBL colour by at most a
  * rounding step. */
@@ -431,8 +449,8 @@ __device__ __forceinline__ void dir_uv(float dx, float dy, float dz, float rot, 
                                        float *v) {
   float phi = atan2f(dz, dx) + rot;
   float cdy = dy < -1.0f ? -1.0f : (dy > 1.0f ? 1.0f : dy);
-  *u = phi / (2.0f * 3.14159265f) + 0.5f;
-  *v = asinf(cdy) / 3.14159265f + 0.5f;
+  *u = div_const(phi, 2.0f * 3.14159265f) + 0.5f;
+  *v = div_const(asinf(cdy), 3.14159265f) + 0.5f;
 }
 
 __device__ void ibl_irr(const FrameArgs &a, V3 n, float out[3]) {
@@ -1493,7 +1511,7 @@ __device__ __forceinline__ void sky_hdr(const FrameArgs &a, int x, int y, float 
   int x0 = (int)fx, y0 = (int)fy;
   x0 = x0 < 0 ? 0 : (x0 > w - 1 ? w - 1 : x0); /* u, v in [0, 1): already inside */
   y0 = y0 < 0 ? 0 : (y0 > h - 1 ? h - 1 : y0);
-  const int x1 = (x0 + 1) % w, y1 = y0 + 1 < h ? y0 + 1 : h - 1;
+  const int x1 = x0 + 1 < w ? x0 + 1 : 0, y1 = y0 + 1 < h ? y0 + 1 : h - 1;
   const float sx = fx - (float)x0, sy = fy - (float)y0;
   const float4 p00 = __ldg(a.sky + (size_t)y0 * w + x0), p10 = __ldg(a.sky + (size_t)y0 * w + x1);
   const float4 p01 = __ldg(a.sky + (size_t)y1 * w + x0), p11 = __ldg(a.sky + (size_t)y1 * w + x1);
@@ -1516,10 +1534,12 @@ __device__ __forceinline__ uchar4 sky_resolved(const FrameArgs &a, uint32_t i) {
 }
 
 /* Writes the background (clear colour resolved with id 0 and depth 1,
- * rasterizer.c:2785-2792) to every sample with 16-byte stores — k_shade
- * overwrites the covered ones — and queues covered samples for shading in
- * sample order (each thread owns 8 consecutive samples; one atomicAdd per
- * block iteration).  Blocks of 256 threads. */
+ * rasterizer.c:2785-2792) with 16-byte stores, except where a warp's 256
+ * samples are all covered (k_shade writes covered samples; leaving out each
+ * covered four instead made the stores diverge: 2 us more at 2 M triangles),
+ * and queues covered samples for shading in sample order (each thread owns 8
+ * consecutive samples; one atomicAdd per block iteration).  Blocks of 256
+ * threads. */
 #define RESOLVE_PER_THREAD 8
 
 /* This thread's 8 keys of the chunk at blk (full chunks only; the ragged
@@ -1567,12 +1587,14 @@ __device__ __forceinline__ void resolve_chunk_keys(const FrameArgs &a, uint32_t 
       uint4 *pc = reinterpret_cast<uint4 *>(a.pre + i0);
       float4 *pd = reinterpret_cast<float4 *>(a.depth + i0);
       uint4 *pi = reinterpret_cast<uint4 *>(a.ids + i0);
-      pc[0] = c4;
-      pc[1] = c4;
-      pd[0] = d4;
-      pd[1] = d4;
-      pi[0] = z4;
-      pi[1] = z4;
+      if (!__all_sync(__activemask(), mask == 0xffu)) {
+        pc[0] = c4;
+        pc[1] = c4;
+        pd[0] = d4;
+        pd[1] = d4;
+        pi[0] = z4;
+        pi[1] = z4;
+      }
     } else {
       for (int k = 0; k < RESOLVE_PER_THREAD; k++) {
         const uint32_t i = i0 + (uint32_t)k;
@@ -1611,10 +1633,17 @@ __device__ __forceinline__ void resolve_chunk_keys(const FrameArgs &a, uint32_t 
       s_base = run ? atomicAdd(&a.ctr->shade_count, run) : 0u;
     }
     __syncthreads();
+    /* entries as y << 16 | x: one division here instead of one per shaded sample */
     uint32_t pos = s_base + s_warp[warp] + incl - c;
-    for (int k = 0; k < RESOLVE_PER_THREAD; k++)
+    uint32_t y = mask ? i0 / (uint32_t)a.width : 0u, x = i0 - y * (uint32_t)a.width;
+    for (int k = 0; k < RESOLVE_PER_THREAD; k++) {
       if ((mask >> k) & 1u)
-        a.shade_list[pos++] = i0 + (uint32_t)k;
+        a.shade_list[pos++] = (y << 16) | x;
+      if (++x == (uint32_t)a.width) {
+        x = 0u;
+        y++;
+      }
+    }
     __syncthreads();
   }
 }
@@ -1684,7 +1713,9 @@ __device__ __forceinline__ const LightRec *stage_lights(const FrameArgs &a, Ligh
 template <bool SH>
 __device__ __forceinline__ void shade_item(const FrameArgs &a, uint32_t j, const LightRec *lights) {
   {
-    const uint32_t px = a.shade_list[j];
+    const uint32_t xy = a.shade_list[j];
+    const int x = (int)(xy & 0xffffu), y = (int)(xy >> 16);
+    const uint32_t px = (uint32_t)y * (uint32_t)a.width + (uint32_t)x;
     const unsigned long long k = a.keys[px];
     const uint32_t t = (uint32_t)k >> ORDER_FAN_BITS;
     const uint32_t fan = (uint32_t)k & ((1u << ORDER_FAN_BITS) - 1u);
@@ -1708,7 +1739,6 @@ __device__ __forceinline__ void shade_item(const FrameArgs &a, uint32_t j, const
       a.ids[px] = 0u;
       return;
     }
-    const int x = (int)(px % (uint32_t)a.width), y = (int)(px / (uint32_t)a.width);
     const ShadeRec s = a.srec[rid];
     const DrawRec &d = a.draws[s.draw < a.draw_count ? s.draw : 0];
     const LightRec *Ls = lights + d.light_off;

@@ -821,22 +821,20 @@ int mc_build_draw(const MopCudaDraw *c, const float *model, const float *mvp,
       memset(&L, 0, sizeof L);
       L.type = s.type;
       memcpy(L.position, s.position, sizeof L.position);
-      memcpy(L.direction, s.direction, sizeof L.direction);
       memcpy(L.color, s.color, sizeof L.color);
       L.intensity = s.intensity;
       L.range = s.range;
       L.spot_inner_cos = s.spot_inner_cos;
       L.spot_outer_cos = s.spot_outer_cos;
-      L.active = s.active;
       /* mop_vec3_normalize(direction) (math.c:43-50), once per frame */
-      float dl = sqrtf(L.direction[0] * L.direction[0] + L.direction[1] * L.direction[1] +
-                       L.direction[2] * L.direction[2]);
+      float dl = sqrtf(s.direction[0] * s.direction[0] + s.direction[1] * s.direction[1] +
+                       s.direction[2] * s.direction[2]);
       if (dl < 1e-8f) {
         L.ndir[0] = L.ndir[1] = L.ndir[2] = 0.0f;
       } else {
         float inv = 1.0f / dl;
         for (int k = 0; k < 3; k++)
-          L.ndir[k] = L.direction[k] * inv;
+          L.ndir[k] = s.direction[k] * inv;
       }
       b[n++] = L;
     }

@@ -80,17 +80,18 @@ struct DrawRec {
   int32_t blend_mode; /* MopBlendMode: 0 opaque, 1 alpha, 2 additive, 3 multiply */
 };
 
-struct LightRec {
-  int32_t type;
+/* An active light, in four 16-byte quarters: the shading loads a quarter at a
+ * time (inactive lights stay out of the list). */
+struct __align__(16) LightRec {
   float position[3];
-  float direction[3];
-  float color[4];
-  float intensity;
+  int32_t type;
+  float ndir[3]; /* mop_vec3_normalize(direction), computed once per frame */
   float range;
+  float color[3];
+  float intensity;
   float spot_inner_cos;
   float spot_outer_cos;
-  int32_t active;
-  float ndir[3]; /* mop_vec3_normalize(direction), computed once per frame */
+  float pad[2];
 };
 
 /* Per fan-triangle raster record, 64 bytes. */
@@ -230,7 +231,7 @@ struct FrameArgs {
   float4 *chunk_w;                  /* the edge values (and the flat depth) at a chunk's first
                                        sample, entries below chunk_cap */
   uint32_t chunk_cap;
-  uint32_t *shade_list;             /* covered sample indices */
+  uint32_t *shade_list;             /* covered samples, y << 16 | x */
   Counters *ctr;
   /* resolve */
   float clear[4];
