@@ -830,8 +830,8 @@ int LaunchCore::enqueue(int parts) {
     }
   launches = sh_launches +
              (uint64_t)mopcuda_launch_batch(a, d_posts.as<PostArgs>(), pv, post_count, post_tiles,
-                                            L, scenes.size() == 1, any_shadow, any_ordered, s,
-                                            parts);
+                                            L, scenes.size() == 1, any_shadow, any_ordered,
+                                            (post_effects & MOPCUDA_POST_FOG) != 0, s, parts);
   CU_TRY(cudaGetLastError());
   if (parts & BATCH_PART_POST) { /* status after the last kernel: read at completion */
     CU_TRY(cudaMemcpyAsync(h_status.p, d_status.p, sizeof(BatchStatus), cudaMemcpyDeviceToHost,

@@ -1857,30 +1857,23 @@ __global__ void __launch_bounds__(256, 4) k_shade(FrameArgs a) {
  * ------------------------------------------------------------------------ */
 #define POST_BX 32
 #define POST_BY 8
+/* Presented pixels a thread filters, one above the other: with one at SSAA 1
+ * the tile's copies, halo and barriers outweighed its 256 samples. */
+template <int SF> struct PostRows {
+  static constexpr int value = SF == 1 ? 4 : 1; /* 20 views' post 290 -> 184 us */
+};
 
 __device__ __forceinline__ float luma(uchar4 p) {
   return 0.299f * (float)p.x + 0.587f * (float)p.y + 0.114f * (float)p.z;
 }
 
-/* FXAA of tile sample (i, j) from its 3x3 neighbourhood in the tile. */
+/* FXAA of tile sample (i, j) past its contrast test (range = mx - mn of the
+ * cross): lM..lE are its cross of lumas, the corners and the blended
+ * neighbour come from the tile. */
 template <int TW>
-__device__ __forceinline__ uchar4 fxaa_tile(const uchar4 (*tc)[TW], const float (*tl)[TW], int i,
-                                            int j) {
-  const uchar4 c = tc[i][j];
-  const float lM = tl[i][j], lN = tl[i - 1][j], lS = tl[i + 1][j], lW = tl[i][j - 1],
-              lE = tl[i][j + 1];
-  float mn = lM, mx = lM;
-  if (lN < mn) mn = lN;
-  if (lS < mn) mn = lS;
-  if (lW < mn) mn = lW;
-  if (lE < mn) mn = lE;
-  if (lN > mx) mx = lN;
-  if (lS > mx) mx = lS;
-  if (lW > mx) mx = lW;
-  if (lE > mx) mx = lE;
-  const float range = mx - mn;
-  if (range < 0.0625f * mx + 0.004f)
-    return c;
+__device__ __forceinline__ uchar4 fxaa_blend(const uchar4 (*tc)[TW], const float (*tl)[TW], int i,
+                                             int j, uchar4 c, float range, float lM, float lN,
+                                             float lS, float lW, float lE) {
   const float lNW = tl[i - 1][j - 1], lNE = tl[i - 1][j + 1], lSW = tl[i + 1][j - 1],
               lSE = tl[i + 1][j + 1];
   const float avg =
@@ -1916,7 +1909,8 @@ __device__ __forceinline__ uchar4 fxaa_tile(const uchar4 (*tc)[TW], const float 
  * asynchronous copies while the current one is filtered. */
 template <int SF> struct PostSmem {
   static constexpr int OX = 4; /* tile column of the block's first own sample */
-  static constexpr int TW = POST_BX * SF + 2 * OX, TH = POST_BY * SF + 2;
+  static constexpr int ROWS = POST_BY * PostRows<SF>::value; /* pixel rows of a tile */
+  static constexpr int TW = POST_BX * SF + 2 * OX, TH = ROWS * SF + 2;
   static constexpr int NBUF = SF <= 3 ? 2 : 1; /* within 48 KB of static shared memory */
   alignas(16) uchar4 c[NBUF][TH][TW];
   float l[TH][TW];
@@ -1959,7 +1953,7 @@ __device__ __forceinline__ void post_fetch(const PostArgs &a, bool vec,
   constexpr int TW = PostSmem<SF>::TW, TH = PostSmem<SF>::TH, OX = PostSmem<SF>::OX;
   const int tid = threadIdx.y * POST_BX + threadIdx.x;
   const int w = a.width, h = a.height;
-  const int sx0 = bx * POST_BX * SF - OX, sy0 = by * POST_BY * SF - 1;
+  const int sx0 = bx * POST_BX * SF - OX, sy0 = by * PostSmem<SF>::ROWS * SF - 1;
   if (vec) {
     for (int i = tid; i < (TW / 4) * TH; i += POST_BX * POST_BY) {
       const int ty = i / (TW / 4), tx = 4 * (i % (TW / 4));
@@ -1987,7 +1981,7 @@ __device__ __forceinline__ void post_luma(const PostArgs &a, bool vec,
   constexpr int TW = PostSmem<SF>::TW, TH = PostSmem<SF>::TH, OX = PostSmem<SF>::OX;
   const int tid = threadIdx.y * POST_BX + threadIdx.x;
   const int w = a.width, h = a.height;
-  const int sx0 = bx * POST_BX * SF - OX, sy0 = by * POST_BY * SF - 1;
+  const int sx0 = bx * POST_BX * SF - OX, sy0 = by * PostSmem<SF>::ROWS * SF - 1;
   if (vec) {
     for (int i = tid; i < (TW / 4) * TH; i += POST_BX * POST_BY) {
       const int ty = i / (TW / 4), tx = 4 * (i % (TW / 4));
@@ -2037,6 +2031,27 @@ __device__ __forceinline__ uint8_t gamma_byte_of(const float *thr, float t) {
   return (uint8_t)n;
 }
 
+/* Vignette, clamp and byte scale of a channel value (postprocess.c:92-112). */
+__device__ __forceinline__ float post_scale(uint32_t fx, float v, float vg) {
+  if (fx & 4u)
+    v *= vg;
+  if (v > 1.0f)
+    v = 1.0f;
+  if (v < 0.0f)
+    v = 0.0f;
+  return v * 255.0f + 0.5f;
+}
+
+__device__ __noinline__ float srgb_pow(float x) {
+  return (float)pow((double)x, (double)(1.0f / 2.4f));
+}
+
+/* A byte taken from the single-precision powf is the one the double-precision
+ * pow gives unless the scaled value lies within this of a whole number: powf
+ * is off by at most 4 ulp (CUDA's error bound), 1.3e-4 here, and the roundings
+ * after it by less than 1e-4. */
+#define POW_MARGIN 1e-3f
+
 /* One sample of the post-process with the FOG bit (postprocess.c:43-112):
  * the byte colour to [0, 1], fog from the sample's depth value, Reinhard,
  * sRGB, vignette, clamp, rounding — the reference's float operations in its
@@ -2044,7 +2059,9 @@ __device__ __forceinline__ uint8_t gamma_byte_of(const float *thr, float t) {
  * search; with vignette the sRGB value itself is needed and powf is taken as
  * the double-precision pow rounded to float (glibc's powf, 0.82 ulp, differs
  * from it by one ulp for 0.06 % of inputs, which moves the byte only when the
- * product lands within that ulp of a rounding boundary). */
+ * product lands within that ulp of a rounding boundary).  The double pow runs
+ * only where powf does not settle the byte: with it for every channel, and the
+ * nine samples unrolled, 2403x1347 samples took 138 us, now 86. */
 __device__ __forceinline__ uchar4 post_fog_sample(const PostArgs &a, const float *thr, uchar4 c,
                                                   float depth, float vg) {
   const uint32_t fx = a.effects;
@@ -2060,7 +2077,7 @@ __device__ __forceinline__ uchar4 post_fog_sample(const PostArgs &a, const float
   uint8_t o[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    float v = (float)in[k] / 255.0f;
+    float v = div_const((float)in[k], 255.0f); /* equal for the 256 bytes */
     v = v + (a.fog_color[k] - v) * factor;
     if (fx & 2u)
       v = v / (v + 1.0f);
@@ -2070,21 +2087,24 @@ __device__ __forceinline__ uchar4 post_fog_sample(const PostArgs &a, const float
     }
     if (fx & 1u) {
       const float x = v > 0.0f ? v : 0.0f;
-      v = x <= 0.0031308f ? x * 12.92f
-                          : 1.055f * (float)pow((double)x, (double)(1.0f / 2.4f)) - 0.055f;
+      if (x <= 0.0031308f) {
+        v = x * 12.92f;
+      } else {
+        const float q = post_scale(fx, 1.055f * powf(x, 1.0f / 2.4f) - 0.055f, vg);
+        const float f = q - floorf(q);
+        if (f > POW_MARGIN && f < 1.0f - POW_MARGIN) {
+          o[k] = u8_of(q);
+          continue;
+        }
+        v = 1.055f * srgb_pow(x) - 0.055f;
+      }
     }
-    if (fx & 4u)
-      v *= vg;
-    if (v > 1.0f)
-      v = 1.0f;
-    if (v < 0.0f)
-      v = 0.0f;
-    o[k] = u8_of(v * 255.0f + 0.5f);
+    o[k] = u8_of(post_scale(fx, v, vg));
   }
   return make_uchar4(o[0], o[1], o[2], c.w);
 }
 
-template <int SF, int TW>
+template <int SF, int TW, bool FOG>
 __device__ __forceinline__ void post_pixel(const PostArgs &a, const uchar4 (*s_c)[TW],
                                            const float (*s_l)[TW], const float *s_lut,
                                            const uint8_t *s_lut8, const float *s_thr, int px,
@@ -2094,7 +2114,7 @@ __device__ __forceinline__ void post_pixel(const PostArgs &a, const uchar4 (*s_c
  * landed: this thread's lumas, a barrier, then each thread's pixel (FXAA,
  * the tonemap/gamma map and the SSAA box).  Block-uniform; ends with a
  * barrier so the caller may refill the buffers. */
-template <int SF>
+template <int SF, bool FOG>
 __device__ __forceinline__ void post_filter(const PostArgs &a, bool vec, PostSmem<SF> &sm, int buf,
                                             int bx, int by) {
   constexpr int TW = PostSmem<SF>::TW;
@@ -2102,91 +2122,142 @@ __device__ __forceinline__ void post_filter(const PostArgs &a, bool vec, PostSme
   __syncthreads();
   const int pw = a.width / SF, ph = a.height / SF;
   const int px = bx * POST_BX + (int)threadIdx.x;
-  const int py = by * POST_BY + (int)threadIdx.y;
+  const int py = by * PostSmem<SF>::ROWS + (int)threadIdx.y * PostRows<SF>::value;
   if (px < pw && py < ph)
-    post_pixel<SF, TW>(a, sm.c[buf], sm.l, sm.lut, sm.lut8, sm.thr, px, py);
+    post_pixel<SF, TW, FOG>(a, sm.c[buf], sm.l, sm.lut, sm.lut8, sm.thr, px, py);
   __syncthreads();
 }
 
 /* One tile of POST_BX x POST_BY presented pixels (bx, by), copied and
  * filtered with nothing in flight around it. */
-template <int SF>
+template <int SF, bool FOG>
 __device__ __forceinline__ void post_tile(const PostArgs &a, PostSmem<SF> &sm, int bx, int by) {
   const bool vec = post_vec(a);
   post_fetch<SF>(a, vec, sm.c[0], bx, by);
   cp_async_wait<0>();
-  post_filter<SF>(a, vec, sm, 0, bx, by);
+  post_filter<SF, FOG>(a, vec, sm, 0, bx, by);
 }
 
-template <int SF, int TW>
+/* The thread's samples (PostRows pixels of SF x SF): for SF 1 and 2 their
+ * lumas and the ring around them (without its corners) and their colours are
+ * read once, two columns at a time for SF 2 (a thread's samples lie SF words
+ * apart, so single words would collide in the banks); most samples end at the
+ * contrast test.  Reading per sample took 67.6 us for 3840x2160 samples at SF
+ * 2 (now 58.4).  FOG in a kernel of its own: with it the others' registers
+ * cost a resident block. */
+template <int SF, int TW, bool FOG>
 __device__ __forceinline__ void post_pixel(const PostArgs &a, const uchar4 (*s_c)[TW],
                                            const float (*s_l)[TW], const float *s_lut,
                                            const uint8_t *s_lut8, const float *s_thr, int px,
                                            int py) {
-  const int w = a.width, h = a.height, pw = w / SF;
+  constexpr int RP = PostRows<SF>::value, N = SF * RP; /* sample rows */
+  constexpr bool WIN = SF <= 2;
+  const int w = a.width, h = a.height, pw = w / SF, ph = h / SF;
   const bool fx = (a.effects & 16u) && w >= 3 && h >= 3;
-  uint32_t acc[4] = {0, 0, 0, 0};
+  const int ti0 = (int)threadIdx.y * N + 1, tj0 = (int)threadIdx.x * SF + PostSmem<SF>::OX;
+  float l[WIN ? N + 2 : 1][WIN ? SF + 2 : 1];
+  uchar4 col[WIN ? N : 1][WIN ? SF : 1];
+  if (WIN) {
 #pragma unroll
-  for (int dy = 0; dy < SF; dy++)
-#pragma unroll
-    for (int dx = 0; dx < SF; dx++) {
-      const int x = px * SF + dx, y = py * SF + dy;
-      const int ti = (int)threadIdx.y * SF + dy + 1,
-                tj = (int)threadIdx.x * SF + dx + PostSmem<SF>::OX;
-      uchar4 c = s_c[ti][tj];
-      if (fx && x >= 1 && y >= 1 && x < w - 1 && y < h - 1)
-        c = fxaa_tile<TW>(s_c, s_l, ti, tj);
-      if (a.effects & 8u) {
-        float vg = 1.0f;
-        if (a.effects & 4u) {
-          const float cx = (float)w * 0.5f, cy = (float)h * 0.5f;
-          const float maxd = sqrtf(cx * cx + cy * cy);
-          const float ddx = (float)x - cx, ddy = (float)y - cy;
-          const float dist = sqrtf(ddx * ddx + ddy * ddy) / maxd;
-          vg = 1.0f - dist * dist * 0.5f;
-          if (vg < 0.0f)
-            vg = 0.0f;
-        }
-        c = post_fog_sample(a, s_thr, c, a.depth[(size_t)y * w + x], vg);
-      } else if (a.effects != 0u && !(a.effects & 4u)) {
-        /* without vignette the post-process is a fixed byte map */
-        c.x = s_lut8[c.x];
-        c.y = s_lut8[c.y];
-        c.z = s_lut8[c.z];
-      } else if (a.effects != 0u) {
-        float v[3] = {s_lut[c.x], s_lut[c.y], s_lut[c.z]};
-        if (a.effects & 4u) {
-          const float cx = (float)w * 0.5f, cy = (float)h * 0.5f;
-          const float maxd = sqrtf(cx * cx + cy * cy);
-          const float ddx = (float)x - cx, ddy = (float)y - cy;
-          const float dist = sqrtf(ddx * ddx + ddy * ddy) / maxd;
-          float vg = 1.0f - dist * dist * 0.5f;
-          if (vg < 0.0f)
-            vg = 0.0f;
-          for (int k = 0; k < 3; k++)
-            v[k] *= vg;
-        }
-        for (int k = 0; k < 3; k++) {
-          if (v[k] > 1.0f)
-            v[k] = 1.0f;
-          if (v[k] < 0.0f)
-            v[k] = 0.0f;
-        }
-        c.x = u8_of(v[0] * 255.0f + 0.5f);
-        c.y = u8_of(v[1] * 255.0f + 0.5f);
-        c.z = u8_of(v[2] * 255.0f + 0.5f);
+    for (int i = 0; i < N + 2; i++) {
+      if (SF == 2) {
+        const float2 v = *reinterpret_cast<const float2 *>(&s_l[ti0 + i - 1][tj0]);
+        l[WIN ? i : 0][WIN ? 1 : 0] = v.x;
+        l[WIN ? i : 0][SF == 2 ? 2 : 0] = v.y;
+      } else {
+        l[WIN ? i : 0][WIN ? 1 : 0] = s_l[ti0 + i - 1][tj0];
       }
-      a.out[(size_t)y * w + x] = c;
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      if (SF == 2) {
+        const uint2 v = *reinterpret_cast<const uint2 *>(&s_c[ti0 + i][tj0]);
+        col[WIN ? i : 0][0] = *reinterpret_cast<const uchar4 *>(&v.x);
+        col[WIN ? i : 0][SF == 2 ? 1 : 0] = *reinterpret_cast<const uchar4 *>(&v.y);
+      } else {
+        col[WIN ? i : 0][0] = s_c[ti0 + i][tj0];
+      }
+      l[WIN ? i + 1 : 0][0] = s_l[ti0 + i][tj0 - 1];
+      l[WIN ? i + 1 : 0][WIN ? SF + 1 : 0] = s_l[ti0 + i][tj0 + SF];
+    }
+  }
+  auto lum = [&](int i, int j) {
+    return WIN ? l[WIN ? i : 0][WIN ? j : 0] : s_l[ti0 + i - 1][tj0 + j - 1];
+  };
+  float maxd = 0.0f;
+  if (a.effects & 4u) {
+    const float cx = (float)w * 0.5f, cy = (float)h * 0.5f;
+    maxd = sqrtf(cx * cx + cy * cy);
+  }
+  auto vignette = [&](int x, int y) {
+    const float cx = (float)w * 0.5f, cy = (float)h * 0.5f;
+    const float ddx = (float)x - cx, ddy = (float)y - cy;
+    const float dist = sqrtf(ddx * ddx + ddy * ddy) / maxd;
+    const float vg = 1.0f - dist * dist * 0.5f;
+    return vg < 0.0f ? 0.0f : vg;
+  };
+  auto sample = [&](int i, int j, int x, int y) { /* row i, column j of the thread's samples */
+    uchar4 c = WIN ? col[WIN ? i : 0][WIN ? j : 0] : s_c[ti0 + i][tj0 + j];
+    if (fx && x >= 1 && y >= 1 && x < w - 1 && y < h - 1) {
+      const float lM = lum(i + 1, j + 1), lN = lum(i, j + 1), lS = lum(i + 2, j + 1),
+                  lW = lum(i + 1, j), lE = lum(i + 1, j + 2);
+      /* lumas are finite and not below +0: min and max in any order */
+      const float mn = fminf(fminf(fminf(lM, lN), fminf(lS, lW)), lE);
+      const float mx = fmaxf(fmaxf(fmaxf(lM, lN), fmaxf(lS, lW)), lE);
+      const float range = mx - mn;
+      if (!(range < 0.0625f * mx + 0.004f))
+        c = fxaa_blend<TW>(s_c, s_l, ti0 + i, tj0 + j, c, range, lM, lN, lS, lW, lE);
+    }
+    if (FOG) {
+      c = post_fog_sample(a, s_thr, c, __ldg(a.depth + (size_t)y * w + x),
+                          (a.effects & 4u) ? vignette(x, y) : 1.0f);
+    } else if (a.effects != 0u && !(a.effects & 4u)) {
+      /* without vignette the post-process is a fixed byte map */
+      c.x = s_lut8[c.x];
+      c.y = s_lut8[c.y];
+      c.z = s_lut8[c.z];
+    } else if (a.effects != 0u) {
+      const float vg = vignette(x, y);
+      float v[3] = {s_lut[c.x] * vg, s_lut[c.y] * vg, s_lut[c.z] * vg};
+      for (int k = 0; k < 3; k++) {
+        if (v[k] > 1.0f)
+          v[k] = 1.0f;
+        if (v[k] < 0.0f)
+          v[k] = 0.0f;
+      }
+      c.x = u8_of(v[0] * 255.0f + 0.5f);
+      c.y = u8_of(v[1] * 255.0f + 0.5f);
+      c.z = u8_of(v[2] * 255.0f + 0.5f);
+    }
+    a.out[(size_t)y * w + x] = c;
+    return c;
+  };
+#pragma unroll
+  for (int r = 0; r < RP; r++) {
+    if (py + r >= ph)
+      break;
+    uint32_t acc[4] = {0, 0, 0, 0};
+    auto add = [&](uchar4 c) {
       acc[0] += c.x;
       acc[1] += c.y;
       acc[2] += c.z;
       acc[3] += c.w;
+    };
+    if (WIN) {
+#pragma unroll
+      for (int k = 0; k < SF * SF; k++)
+        add(sample(r * SF + k / SF, k % SF, px * SF + k % SF, (py + r) * SF + k / SF));
+    } else { /* unrolled, the nine or sixteen samples' code outgrows the instruction cache */
+#pragma unroll 1
+      for (int k = 0; k < SF * SF; k++)
+        add(sample(r * SF + k / SF, k % SF, px * SF + k % SF, (py + r) * SF + k / SF));
     }
-  if (a.presented) {
-    const uint32_t n = (uint32_t)(SF * SF);
-    a.presented[(size_t)py * pw + px] =
-        make_uchar4((uint8_t)(acc[0] / n), (uint8_t)(acc[1] / n), (uint8_t)(acc[2] / n),
-                    (uint8_t)(acc[3] / n));
+    if (a.presented) {
+      const uint32_t n = (uint32_t)(SF * SF);
+      a.presented[(size_t)(py + r) * pw + px] =
+          make_uchar4((uint8_t)(acc[0] / n), (uint8_t)(acc[1] / n), (uint8_t)(acc[2] / n),
+                      (uint8_t)(acc[3] / n));
+    }
   }
 }
 
@@ -2194,18 +2265,19 @@ __device__ __forceinline__ void post_pixel(const PostArgs &a, const uchar4 (*s_c
  * blockIdx.x + gridDim.x, ... in row-major tile order; with two colour
  * buffers the copies of the next tile are in flight while the current one
  * is filtered. */
-template <int SF>
+template <int SF, bool FOG>
 __global__ void __launch_bounds__(POST_BX *POST_BY) k_post(PostArgs a) {
   pdl_wait();
   __shared__ PostSmem<SF> sm;
   post_load_luts<SF>(a, sm);
   const bool vec = post_vec(a);
   const uint32_t tx = ((uint32_t)(a.width / SF) + POST_BX - 1u) / POST_BX;
-  const uint32_t ty = ((uint32_t)(a.height / SF) + POST_BY - 1u) / POST_BY;
+  const uint32_t ty =
+      ((uint32_t)(a.height / SF) + PostSmem<SF>::ROWS - 1u) / PostSmem<SF>::ROWS;
   const uint32_t nt = tx * ty;
   if (PostSmem<SF>::NBUF == 1) {
     for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x)
-      post_tile<SF>(a, sm, (int)(t % tx), (int)(t / tx));
+      post_tile<SF, FOG>(a, sm, (int)(t % tx), (int)(t / tx));
     return;
   }
   uint32_t t = blockIdx.x;
@@ -2220,15 +2292,15 @@ __global__ void __launch_bounds__(POST_BX *POST_BY) k_post(PostArgs a) {
     } else {
       cp_async_wait<0>();
     }
-    post_filter<SF>(a, vec, sm, buf & (PostSmem<SF>::NBUF - 1), (int)(t % tx), (int)(t / tx));
+    post_filter<SF, FOG>(a, vec, sm, buf & (PostSmem<SF>::NBUF - 1), (int)(t % tx), (int)(t / tx));
   }
 }
 
 /* Blocks of k_post<SF> resident on one SM (queried once per factor). */
-template <int SF> static int post_resident() {
+template <int SF, bool FOG> static int post_resident() {
   static int nb = 0;
   if (nb == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_post<SF>, POST_BX * POST_BY, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_post<SF, FOG>, POST_BX * POST_BY, 0) !=
             cudaSuccess ||
         nb < 1) {
       cudaGetLastError();
@@ -2237,11 +2309,6 @@ template <int SF> static int post_resident() {
   }
   return nb;
 }
-
-template __global__ void k_post<1>(PostArgs);
-template __global__ void k_post<2>(PostArgs);
-template __global__ void k_post<3>(PostArgs);
-template __global__ void k_post<4>(PostArgs);
 
 /* SSAA box of an already post-processed buffer (read_color path). */
 __global__ void k_box(const uchar4 *src, int width, int height, int sf, uchar4 *dst) {
@@ -2421,23 +2488,30 @@ int mopcuda_launch_frame(const FrameArgs &a, const PostArgs &p, const LaunchCfg 
   const int sf = p.ssaa;
   dim3 pb(POST_BX, POST_BY);
   const uint32_t tiles = blocks_for((uint32_t)(p.width / sf), POST_BX) *
-                         blocks_for((uint32_t)(p.height / sf), POST_BY);
+                         blocks_for((uint32_t)(p.height / sf),
+                                    POST_BY * (sf == 1 ? PostRows<1>::value : 1));
   auto pgrid = [&](int resident) {
     const uint32_t g = (uint32_t)cfg.num_sms * (uint32_t)resident;
     return tiles < g ? (tiles ? tiles : 1u) : g;
   };
+  auto post = [&](auto k, int resident) { pdl(k, pgrid(resident), pb, s, p); };
+  const bool fog = (p.effects & 8u) != 0;
   switch (sf) {
   case 2:
-    pdl(k_post<2>, pgrid(post_resident<2>()), pb, s, p);
+    fog ? post(k_post<2, true>, post_resident<2, true>())
+        : post(k_post<2, false>, post_resident<2, false>());
     break;
   case 3:
-    pdl(k_post<3>, pgrid(post_resident<3>()), pb, s, p);
+    fog ? post(k_post<3, true>, post_resident<3, true>())
+        : post(k_post<3, false>, post_resident<3, false>());
     break;
   case 4:
-    pdl(k_post<4>, pgrid(post_resident<4>()), pb, s, p);
+    fog ? post(k_post<4, true>, post_resident<4, true>())
+        : post(k_post<4, false>, post_resident<4, false>());
     break;
   default:
-    pdl(k_post<1>, pgrid(post_resident<1>()), pb, s, p);
+    fog ? post(k_post<1, true>, post_resident<1, true>())
+        : post(k_post<1, false>, post_resident<1, false>());
     break;
   }
   launches++;
@@ -3954,11 +4028,11 @@ __global__ void __launch_bounds__(32 * WLONG_WARPS) k_b_wlong(const FrameArgs *_
 template <int SF>
 __device__ __forceinline__ uint32_t post_tiles_of(const PostArgs &p) {
   const uint32_t pw = (uint32_t)(p.width / SF), ph = (uint32_t)(p.height / SF);
-  return ((pw + POST_BX - 1u) / POST_BX) * ((ph + POST_BY - 1u) / POST_BY);
+  return ((pw + POST_BX - 1u) / POST_BX) * ((ph + PostSmem<SF>::ROWS - 1u) / PostSmem<SF>::ROWS);
 }
 
 /* Post tiles of the viewports listed in views (all with ssaa SF). */
-template <int SF>
+template <int SF, bool FOG>
 __global__ void __launch_bounds__(POST_BX *POST_BY, 4) k_b_post(const PostArgs *__restrict__ posts,
                                                              const uint32_t *__restrict__ views,
                                                              uint32_t n) {
@@ -3983,17 +4057,46 @@ __global__ void __launch_bounds__(POST_BX *POST_BY, 4) k_b_post(const PostArgs *
     if (tid == 0)
       s_pre[n] = run;
   }
+  if (n)
+    post_load_luts<SF>(posts[views[0]], sm); /* one set of effects per launch */
   __syncthreads();
   const uint32_t total = s_pre[n];
-  uint32_t k = 0;
-  for (uint32_t u = blockIdx.x; u < total; u += gridDim.x) {
+  /* tile u as its viewport and place; k: the viewport of an earlier tile */
+  auto at = [&](uint32_t u, uint32_t &k, int &bx, int &by) -> const PostArgs & {
     while (s_pre[k + 1] <= u)
       k++;
     const PostArgs &p = posts[views[k]];
-    const uint32_t local = u - s_pre[k];
     const uint32_t tx = ((uint32_t)(p.width / SF) + POST_BX - 1u) / POST_BX;
-    post_load_luts<SF>(p, sm);
-    post_tile<SF>(p, sm, (int)(local % tx), (int)(local / tx));
+    bx = (int)((u - s_pre[k]) % tx);
+    by = (int)((u - s_pre[k]) / tx);
+    return p;
+  };
+  uint32_t k = 0, u = blockIdx.x;
+  int bx = 0, by = 0;
+  if (PostSmem<SF>::NBUF == 1) {
+    for (; u < total; u += gridDim.x) {
+      const PostArgs &p = at(u, k, bx, by);
+      post_tile<SF, FOG>(p, sm, bx, by);
+    }
+    return;
+  }
+  /* as k_post: the next tile's copies are in flight while one is filtered */
+  if (u < total) {
+    const PostArgs &p = at(u, k, bx, by);
+    post_fetch<SF>(p, post_vec(p), sm.c[0], bx, by);
+  }
+  for (int buf = 0; u < total; u += gridDim.x, buf ^= 1) {
+    const PostArgs &p = at(u, k, bx, by);
+    if (u + gridDim.x < total) {
+      uint32_t kn = k;
+      int nx, ny;
+      const PostArgs &q = at(u + gridDim.x, kn, nx, ny);
+      post_fetch<SF>(q, post_vec(q), sm.c[buf ^ (PostSmem<SF>::NBUF - 1)], nx, ny);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    post_filter<SF, FOG>(p, post_vec(p), sm, buf & (PostSmem<SF>::NBUF - 1), bx, by);
   }
 }
 
@@ -4021,7 +4124,7 @@ void mopcuda_batch_grids(BatchLaunch &cfg) {
 int mopcuda_launch_batch(const BatchArgs &b, const PostArgs *posts, const uint32_t *post_views[4],
                          const uint32_t post_count[4], const uint32_t post_tiles[4],
                          const BatchLaunch &cfg, bool shared_lights, bool shadows, bool ordered,
-                         cudaStream_t s, int parts) {
+                         bool fog, cudaStream_t s, int parts) {
   if (b.nv == 0)
     return 0;
   int launches = 0;
@@ -4083,19 +4186,23 @@ int mopcuda_launch_batch(const BatchArgs &b, const PostArgs *posts, const uint32
   for (int k = 0; k < 4; k++) {
     if (!post_count[k] || !post_tiles[k])
       continue;
-    const uint32_t g = post_tiles[k] < (uint32_t)(sms * 16) ? post_tiles[k] : (uint32_t)(sms * 16);
+    const uint32_t g = post_tiles[k] < (uint32_t)(sms * 4) ? post_tiles[k] : (uint32_t)(sms * 4);
     switch (k + 1) {
     case 1:
-      k_b_post<1><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
+      fog ? k_b_post<1, true><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k])
+          : k_b_post<1, false><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
       break;
     case 2:
-      k_b_post<2><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
+      fog ? k_b_post<2, true><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k])
+          : k_b_post<2, false><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
       break;
     case 3:
-      k_b_post<3><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
+      fog ? k_b_post<3, true><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k])
+          : k_b_post<3, false><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
       break;
     default:
-      k_b_post<4><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
+      fog ? k_b_post<4, true><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k])
+          : k_b_post<4, false><<<g, pb, 0, s>>>(posts, post_views[k], post_count[k]);
       break;
     }
     launches++;

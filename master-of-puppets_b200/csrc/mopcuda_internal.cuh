@@ -551,11 +551,12 @@ void mopcuda_batch_grids(BatchLaunch &cfg);
 #define BATCH_PART_MAIN 1
 #define BATCH_PART_POST 2
 /* ordered: the launch has suffix buffers (b.hdr): the suffix kernels run
- * after shading for the viewports that have a suffix. */
+ * after shading for the viewports that have a suffix.  fog: the posts' effects
+ * have the FOG bit. */
 int mopcuda_launch_batch(const BatchArgs &b, const PostArgs *posts, const uint32_t *post_views[4],
                          const uint32_t post_count[4], const uint32_t post_tiles[4],
                          const BatchLaunch &cfg, bool shared_lights, bool shadows, bool ordered,
-                         cudaStream_t s, int parts = BATCH_PART_MAIN | BATCH_PART_POST);
+                         bool fog, cudaStream_t s, int parts = BATCH_PART_MAIN | BATCH_PART_POST);
 
 /* ev (optional, 7 events): stage boundaries
  * vertex | setup+clip | raster | resolve | shade | post */
