@@ -31,7 +31,9 @@
  * completed and its writes are visible (griddepcontrol.wait).  A kernel
  * launched without the attribute passes pdl_wait() at once, so the kernels
  * stay correct wherever they are launched from.  No kernel triggers early:
- * a successor starts once all of its predecessor's blocks have exited. */
+ * a successor starts once all of its predecessor's blocks have exited.
+ * (Triggering after the wait, so that successors' blocks take the room as it
+ * comes free, made every frame 6-9 % slower.) */
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename Arg>
@@ -787,53 +789,70 @@ __device__ __forceinline__ uint32_t rec_chunks(const RasterRec &r) {
   return ((uint32_t)r.x1 - (uint32_t)r.x0) / RASTER_CHUNK + 1u;
 }
 
-/* Queues a large record: one 64-bit atomic takes its list slot (high word)
- * and the offset of its first item (low word) together, so the offsets come
- * out ascending with the slot and no scan pass is needed.  (An atomic per
- * record: the setup of 20 views with many large records took 155 us, with the
- * table's counter 290; with the group's shared ones 90.)  An item total
- * past 2^32 carries into the slot count: flagged (bit 9), the frame fails.
- * Its chunk_w entries are taken too; past the capacity it has none. */
+/* Takes a list slot and the offset of its n items together: one 64-bit atomic
+ * on the list's (items, count) counter pair, so the offsets come out
+ * ascending with the slots and no scan pass is needed.  The converged lanes
+ * with the same pair share the atomic: one lane adds the group's total and
+ * each takes its place behind the lanes below it, as it does behind `extra`,
+ * whose group sum goes to *extra_count when given.  (An atomic per record: the
+ * setup of 20 views with many large records took 155 us, with the chunk
+ * table's counter 290; with the group's shared ones 90.)  An item total past
+ * 2^32 carries into the count: flagged (bit 9), the frame fails. */
+struct ListPlace {
+  uint32_t slot, off;
+  unsigned long long extra;
+};
+__device__ __forceinline__ ListPlace push_items(const FrameArgs &a, uint32_t *pair, uint32_t n,
+                                                uint32_t extra,
+                                                unsigned long long *extra_count) {
+  const uint32_t mask = __activemask(), lane = threadIdx.x & 31u;
+  const uint32_t peers = __match_any_sync(mask, (unsigned long long)(uintptr_t)pair);
+  uint32_t before_n = 0, sum_n = 0, before_e = 0, sum_e = 0;
+  for (uint32_t m = peers; m; m &= m - 1u) {
+    const uint32_t src = (uint32_t)__ffs((int)m) - 1u;
+    const uint32_t vn = __shfl_sync(peers, n, (int)src);
+    before_n += src < lane ? vn : 0u;
+    sum_n += vn;
+    if (extra_count) {
+      const uint32_t ve = __shfl_sync(peers, extra, (int)src);
+      before_e += src < lane ? ve : 0u;
+      sum_e += ve;
+    }
+  }
+  const int leader = __ffs((int)peers) - 1;
+  unsigned long long old = 0, e = 0;
+  if ((int)lane == leader) {
+    old = atomicAdd(reinterpret_cast<unsigned long long *>(pair),
+                    ((unsigned long long)__popc(peers) << 32) | sum_n);
+    if (extra_count)
+      e = atomicAdd(extra_count, (unsigned long long)sum_e);
+  }
+  old = __shfl_sync(peers, old, leader);
+  if (extra_count)
+    e = __shfl_sync(peers, e, leader);
+  if ((uint32_t)old + sum_n < sum_n)
+    atomicOr(&a.ctr->overflow, 512u);
+  ListPlace p;
+  p.slot = (uint32_t)(old >> 32) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  p.off = (uint32_t)old + before_n;
+  p.extra = e + before_e;
+  return p;
+}
+
+/* Queues a large record and takes its chunk_w entries (past the capacity it
+ * has none). */
 __device__ __forceinline__ void push_large(const FrameArgs &a, uint32_t rid, const RasterRec &r) {
   const uint32_t h = (uint32_t)(r.y1 & 0x7fffu) - (uint32_t)r.y0 + 1u, chunks = rec_chunks(r);
   const bool wide = chunks > WIDE_CHUNKS;
   const uint32_t n = wide ? (h + BAND_ROWS - 1u) / BAND_ROWS *
                                 ((chunks + BAND_CHUNKS - 1u) / BAND_CHUNKS)
                           : h;
-  /* the converged lanes with the same list share the atomics: one lane adds
-   * the group's total and each takes its place behind the lanes below it */
-  const uint32_t mask = __activemask(), lane = threadIdx.x & 31u;
-  const uint32_t peers =
-      __match_any_sync(mask, (unsigned long long)(uintptr_t)a.ctr + (wide ? 1u : 0u));
-  uint32_t before_n = 0, sum_n = 0, before_e = 0, sum_e = 0;
-  for (uint32_t m = peers; m; m &= m - 1u) {
-    const uint32_t src = (uint32_t)__ffs((int)m) - 1u;
-    const uint32_t vn = __shfl_sync(peers, n, (int)src);
-    const uint32_t ve = __shfl_sync(peers, h * chunks, (int)src);
-    before_n += src < lane ? vn : 0u;
-    before_e += src < lane ? ve : 0u;
-    sum_n += vn;
-    sum_e += ve;
-  }
-  const int leader = __ffs((int)peers) - 1;
-  unsigned long long old = 0, e = 0;
-  if ((int)lane == leader) {
-    old = atomicAdd(reinterpret_cast<unsigned long long *>(wide ? &a.ctr->wide_items
-                                                                : &a.ctr->large_items),
-                    ((unsigned long long)__popc(peers) << 32) | sum_n);
-    e = atomicAdd(&a.ctr->chunk_count, (unsigned long long)sum_e);
-  }
-  old = __shfl_sync(peers, old, leader);
-  e = __shfl_sync(peers, e, leader);
-  const uint32_t q = (uint32_t)(old >> 32) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-  const uint32_t off = (uint32_t)old + before_n;
-  if ((uint32_t)old + sum_n < sum_n)
-    atomicOr(&a.ctr->overflow, 512u);
-  e += before_e;
-  a.large_off[rid] = e + h * chunks <= a.chunk_cap ? (uint32_t)e : 0xffffffffu;
-  if (q < a.large_cap) {
-    (wide ? a.wide_list : a.large_list)[q] = rid;
-    (wide ? a.wide_items : a.large_items)[q] = off;
+  const ListPlace p = push_items(a, wide ? &a.ctr->wide_items : &a.ctr->large_items, n,
+                                 h * chunks, &a.ctr->chunk_count);
+  a.large_off[rid] = p.extra + h * chunks <= a.chunk_cap ? (uint32_t)p.extra : 0xffffffffu;
+  if (p.slot < a.large_cap) {
+    (wide ? a.wide_list : a.large_list)[p.slot] = rid;
+    (wide ? a.wide_items : a.large_items)[p.slot] = p.off;
   } else {
     atomicOr(&a.ctr->overflow, 8u);
   }
@@ -2362,11 +2381,9 @@ __global__ void k_pick(const uint32_t *ids, const float *depth, int width, int h
 static inline unsigned blocks_for(uint32_t n, unsigned bs) { return (n + bs - 1u) / bs; }
 
 __global__ void k_ocount(FrameArgs a);
-__global__ void k_oscan(FrameArgs a);
 __global__ void k_oraster(FrameArgs a);
 template <bool SH, bool WIRE> __global__ void k_ofold(FrameArgs a);
 __global__ void k_wcount(FrameArgs a);
-__global__ void k_wscan(FrameArgs a);
 __global__ void k_wplot(FrameArgs a);
 #define WLONG_WARPS 4 /* warps of a k_wlong block */
 template <bool SH> __global__ void k_wlong(FrameArgs a);
@@ -2456,14 +2473,12 @@ int mopcuda_launch_frame(const FrameArgs &a, const PostArgs &p, const LaunchCfg 
     cudaMemsetAsync(a.frag_head, 0xff, sizeof(uint32_t) * (size_t)S, s);
     const uint32_t nrec = a.rec_cap < (1u << 22) ? a.rec_cap : (1u << 22);
     pdl(k_ocount, blocks_for(nrec, 256), 256, s, a);
-    pdl(k_oscan, 1, 1024, s, a);
     pdl(k_oraster, cfg.num_sms * 8, 256, s, a);
-    launches += 3;
+    launches += 2;
     if (a.wire) { /* wireframe draws: their line plots join the fragment lists */
       pdl(k_wcount, blocks_for(nrec, 256), 256, s, a);
-      pdl(k_wscan, 1, 1024, s, a);
       pdl(k_wplot, cfg.num_sms * 8, 256, s, a);
-      launches += 3;
+      launches += 2;
       if (a.shadow_keys) {
         pdl(k_ofold<true, true>, cfg.num_sms * 8, 128, s, a);
         pdl(k_wlong<true>, cfg.num_sms * 4, 32 * WLONG_WARPS, s, a);
@@ -2581,20 +2596,23 @@ int mopcuda_launch_pick(const uint32_t *ids, const float *depth, int width, int 
  * depth only decreases), each sample sorts its list by submission order and
  * folds it sequentially.
  * ======================================================================== */
+/* Records that may belong to the suffix: the triangles from t_split on and
+ * the clipped fans. */
 __device__ __forceinline__ uint32_t ordered_record_items(const FrameArgs &a) {
-  return raster_small_items(a);
+  const uint32_t n = raster_small_items(a), t0 = min(a.t_split, a.total_tris);
+  return n > t0 ? n - t0 : 0u;
 }
 
-/* Queues record rid if it is a live record of the suffix, with its
- * (row, chunk) count. */
-__device__ __forceinline__ void ocount_item(const FrameArgs &a, uint32_t rid) {
+/* Queues suffix record i if it is live, with its (row, chunk) items. */
+__device__ __forceinline__ void ocount_item(const FrameArgs &a, uint32_t i) {
+  const uint32_t rid = min(a.t_split, a.total_tris) + i;
   const RasterRec r = a.rrec[rid];
   if (!rec_live(r, a.width, a.height) || !rec_ordered(a, r))
     return;
-  const uint32_t q = atomicAdd(&a.ctr->olist_count, 1u);
-  if (q < a.olist_cap) {
-    a.olist[q] = rid;
-    a.olist_items[q] = rec_items(r);
+  const ListPlace p = push_items(a, &a.ctr->olist_items, rec_items(r), 0u, nullptr);
+  if (p.slot < a.olist_cap) {
+    a.olist[p.slot] = rid;
+    a.olist_items[p.slot] = p.off;
   } else {
     atomicOr(&a.ctr->overflow, 32u);
   }
@@ -2603,18 +2621,8 @@ __device__ __forceinline__ void ocount_item(const FrameArgs &a, uint32_t rid) {
 __global__ void __launch_bounds__(256) k_ocount(FrameArgs a) {
   pdl_wait();
   const uint32_t n = ordered_record_items(a);
-  for (uint32_t rid = blockIdx.x * blockDim.x + threadIdx.x; rid < n;
-       rid += gridDim.x * blockDim.x)
-    ocount_item(a, rid);
-}
-
-__global__ void __launch_bounds__(1024) k_oscan(FrameArgs a) {
-  pdl_wait();
-  __shared__ uint32_t part[32];
-  uint32_t n = a.ctr->olist_count;
-  if (n > a.olist_cap)
-    n = a.olist_cap;
-  items_scan_block(a.olist_items, n, &a.ctr->olist_items, part);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    ocount_item(a, i);
 }
 
 /* Links a fragment into sample px's list.  Node and touched-list slots come
@@ -2841,8 +2849,9 @@ __device__ __forceinline__ unsigned long long frag_key(const FrameArgs &a, uint3
   return ((unsigned long long)k.x << 32) | (unsigned long long)k.y;
 }
 
-/* Queues the live wireframe records of the suffix with their plot counts. */
-__device__ __forceinline__ void wcount_item(const FrameArgs &a, uint32_t rid) {
+/* Queues the live wireframe records of the suffix with their plots. */
+__device__ __forceinline__ void wcount_item(const FrameArgs &a, uint32_t i) {
+  const uint32_t rid = min(a.t_split, a.total_tris) + i;
   const RasterRec r = a.rrec[rid];
   if (r.x1 != (uint16_t)REC_WIRE_X1 || r.y0 == REC_REDIRECT)
     return;
@@ -2852,10 +2861,10 @@ __device__ __forceinline__ void wcount_item(const FrameArgs &a, uint32_t rid) {
     wu_edge(r, e, L);
     n += wu_plots(L);
   }
-  const uint32_t q = atomicAdd(&a.ctr->wire_count, 1u);
-  if (q < a.wlist_cap) {
-    a.wlist[q] = rid;
-    a.wlist_items[q] = n;
+  const ListPlace p = push_items(a, &a.ctr->wire_items, n, 0u, nullptr);
+  if (p.slot < a.wlist_cap) {
+    a.wlist[p.slot] = rid;
+    a.wlist_items[p.slot] = p.off;
   } else {
     atomicOr(&a.ctr->overflow, 128u);
   }
@@ -2867,15 +2876,6 @@ __global__ void __launch_bounds__(256) k_wcount(FrameArgs a) {
   for (uint32_t rid = blockIdx.x * blockDim.x + threadIdx.x; rid < n;
        rid += gridDim.x * blockDim.x)
     wcount_item(a, rid);
-}
-
-__global__ void __launch_bounds__(1024) k_wscan(FrameArgs a) {
-  pdl_wait();
-  __shared__ uint32_t part[32];
-  uint32_t n = a.ctr->wire_count;
-  if (n > a.wlist_cap)
-    n = a.wlist_cap;
-  items_scan_block(a.wlist_items, n, &a.ctr->wire_items, part);
 }
 
 /* One line plot: in the framebuffer, coverage at least 0.004 and in front
@@ -3926,8 +3926,7 @@ __global__ void __launch_bounds__(256, 4) k_b_shade(const FrameArgs *__restrict_
 }
 
 /* The ordered suffix of every viewport that has one, as the single-frame
- * kernels run it: queue the suffix records, scan their item counts (a block
- * per viewport), rasterise them into fragment lists, fold each touched
+ * kernels run it: queue the suffix records, rasterise them into fragment lists, fold each touched
  * sample's list in submission order. */
 __global__ void __launch_bounds__(256) k_b_ocount(const FrameArgs *__restrict__ fr, uint32_t nv) {
   __shared__ uint32_t s_pre[MOPCUDA_MAX_VIEWS + 1];
@@ -3939,13 +3938,6 @@ __global__ void __launch_bounds__(256) k_b_ocount(const FrameArgs *__restrict__ 
       v++;
     ocount_item(fr[v], g - s_pre[v]);
   }
-}
-
-__global__ void __launch_bounds__(1024) k_b_oscan(const FrameArgs *__restrict__ fr) {
-  __shared__ uint32_t part[32];
-  const FrameArgs &a = fr[blockIdx.x];
-  if (a.hdr)
-    items_scan_block(a.olist_items, olist_len(a), &a.ctr->olist_items, part);
 }
 
 __global__ void __launch_bounds__(256) k_b_oraster(const FrameArgs *__restrict__ fr, uint32_t nv) {
@@ -3961,8 +3953,8 @@ __global__ void __launch_bounds__(256) k_b_oraster(const FrameArgs *__restrict__
   }
 }
 
-/* Wireframe records of the viewports that have them (k_wcount, k_wscan,
- * k_wplot per viewport). */
+/* Wireframe records of the viewports that have them (k_wcount and k_wplot
+ * per viewport). */
 __global__ void __launch_bounds__(256) k_b_wcount(const FrameArgs *__restrict__ fr, uint32_t nv) {
   __shared__ uint32_t s_pre[MOPCUDA_MAX_VIEWS + 1];
   const uint32_t total = views_prefix<ST_WCOUNT>(fr, nv, s_pre);
@@ -3972,17 +3964,6 @@ __global__ void __launch_bounds__(256) k_b_wcount(const FrameArgs *__restrict__ 
     while (s_pre[v + 1] <= g)
       v++;
     wcount_item(fr[v], g - s_pre[v]);
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_b_wscan(const FrameArgs *__restrict__ fr) {
-  __shared__ uint32_t part[32];
-  const FrameArgs &a = fr[blockIdx.x];
-  if (a.hdr && a.wire) {
-    uint32_t n = a.ctr->wire_count;
-    if (n > a.wlist_cap)
-      n = a.wlist_cap;
-    items_scan_block(a.wlist_items, n, &a.ctr->wire_items, part);
   }
 }
 
@@ -4157,14 +4138,12 @@ int mopcuda_launch_batch(const BatchArgs &b, const PostArgs *posts, const uint32
     if (ordered && b.hdr) {
       cudaMemsetAsync(b.frag_head, 0xff, sizeof(uint32_t) * (size_t)b.samples, s);
       k_b_ocount<<<sms * 8, 256, 0, s>>>(fr, nv);
-      k_b_oscan<<<nv, 1024, 0, s>>>(fr);
       k_b_oraster<<<sms * 8, 256, 0, s>>>(fr, nv);
-      launches += 4;
+      launches += 3;
       if (b.wlist) { /* some viewport has wireframe draws */
         k_b_wcount<<<sms * 8, 256, 0, s>>>(fr, nv);
-        k_b_wscan<<<nv, 1024, 0, s>>>(fr);
         k_b_wplot<<<sms * 8, 256, 0, s>>>(fr, nv);
-        launches += 3;
+        launches += 2;
         if (shadows) {
           k_b_ofold<true, true><<<sms * 8, 128, 0, s>>>(fr, nv);
           k_b_wlong<true><<<sms * 4, 32 * WLONG_WARPS, 0, s>>>(fr, nv);

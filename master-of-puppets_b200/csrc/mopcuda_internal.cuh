@@ -153,23 +153,26 @@ struct alignas(8) Counters {
   uint32_t wide_count;
   uint32_t clip_count;
   uint32_t overflow;          /* bit0 records, bit1 extra vertices, bit2 clip
-                                 queue, bit3 large list, bit9 large-record
-                                 items past 2^32                               */
+                                 queue, bit3 large list, bit9 a record
+                                 list's items past 2^32                        */
   uint32_t shade_count;       /* covered samples queued for shading              */
+  uint32_t shade_next;        /* samples of the shading list handed out          */
   /* ordered (blended) suffix of the frame; overflow bit4 fragment pool,
    * bit5 ordered-record list, bit7 wireframe-record list */
-  uint32_t frag_count, touched_count, olist_count, olist_items;
-  uint32_t wire_count, wire_items; /* wireframe records queued, their plots */
+  uint32_t frag_count, touched_count;
+  uint32_t olist_items, olist_count; /* pair: suffix records queued, their items */
+  uint32_t wire_items, wire_count;   /* pair: wireframe records queued, their plots */
   uint32_t scratch_count;          /* sort-scratch entries taken by long lists */
   uint32_t wlong_count;            /* samples of wireframe frames with a long list */
-  uint32_t shade_next;             /* samples of the shading list handed out */
   unsigned long long chunk_count;  /* chunk_w entries asked for by large records */
 };
 /* arrays of counters (one per viewport) keep the 64-bit pair aligned */
 static_assert(sizeof(Counters) % 8 == 0 && offsetof(Counters, large_items) % 8 == 0 &&
                   offsetof(Counters, wide_items) % 8 == 0 &&
+                  offsetof(Counters, olist_items) % 8 == 0 &&
+                  offsetof(Counters, wire_items) % 8 == 0 &&
                   offsetof(Counters, chunk_count) % 8 == 0,
-              "large-record counter pairs must be 8-byte aligned");
+              "counter pairs must be 8-byte aligned");
 
 /* Blended fragments of one sample sorted in registers; a sample with more
  * sorts its list in the fold's global scratch (heapsort). */
@@ -263,7 +266,7 @@ struct FrameArgs {
   uint32_t frag_cap;
   uint32_t *touched;      /* samples that received a fragment                   */
   uint32_t *olist;        /* live records of the suffix                          */
-  uint32_t *olist_items;  /* their (row, chunk) item counts, then offsets        */
+  uint32_t *olist_items;  /* offset of each one's first (row, chunk) item        */
   uint32_t olist_cap;
   /* environment background (pass_background_hdri_cpu): every uncovered
    * sample shows the RGBA32F environment (sky_w x sky_h) along the ray
@@ -277,8 +280,8 @@ struct FrameArgs {
    * depth, and later ones may pass where the opaque depth is nearer, so
    * every covered fragment of the suffix is kept */
   int ordered_keep_all;
-  /* wireframe records in the suffix: their queue and plot counts (then
-   * offsets); wire != 0 when the frame has wireframe draws */
+  /* wireframe records in the suffix: their queue and first plots' offsets;
+   * wire != 0 when the frame has wireframe draws */
   uint32_t *wlist, *wlist_items;
   uint32_t wlist_cap;
   int wire;
