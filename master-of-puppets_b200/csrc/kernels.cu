@@ -759,6 +759,24 @@ __device__ __forceinline__ uint32_t warp_alloc1(uint32_t *counter) {
   return base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
 }
 
+/* The same for n slots per lane. */
+__device__ __forceinline__ uint32_t warp_alloc(uint32_t *counter, uint32_t n) {
+  const uint32_t mask = __activemask(), lane = threadIdx.x & 31u;
+  const uint32_t peers = __match_any_sync(mask, (unsigned long long)(uintptr_t)counter);
+  uint32_t before = 0, sum = 0;
+  for (uint32_t m = peers; m; m &= m - 1u) {
+    const uint32_t src = (uint32_t)__ffs((int)m) - 1u;
+    const uint32_t v = __shfl_sync(peers, n, (int)src);
+    before += src < lane ? v : 0u;
+    sum += v;
+  }
+  const int leader = __ffs((int)peers) - 1;
+  uint32_t base = 0;
+  if ((int)lane == leader)
+    base = atomicAdd(counter, sum);
+  return __shfl_sync(peers, base, leader) + before;
+}
+
 __device__ __forceinline__ bool rec_live(const RasterRec &r, int W, int H) {
   int y1 = (int)(r.y1 & 0x7fffu);
   /* live records always lie inside the framebuffer; anything else is dead
@@ -2644,6 +2662,41 @@ __device__ __forceinline__ uint32_t push_fragment(const FrameArgs &a, uint32_t p
   return node;
 }
 
+/* Fragments of one record at samples row + i for the bits i of m. */
+__device__ __forceinline__ void push_fragments(const FrameArgs &a, uint32_t row, uint32_t m,
+                                               uint32_t order) {
+  uint32_t node = warp_alloc(&a.ctr->frag_count, (uint32_t)__popc(m));
+  uint32_t fresh = 0; /* bits whose sample had no fragment yet */
+  while (m) {
+    uint32_t bit[4], prev[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      bit[k] = m & (0u - m); /* lowest, 0 when none is left */
+      m ^= bit[k];
+      if (bit[k] && node + k < a.frag_cap)
+        prev[k] = atomicExch(&a.frag_head[row + (uint32_t)__ffs((int)bit[k]) - 1u], node + k);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (!bit[k])
+        break;
+      if (node + k >= a.frag_cap) {
+        atomicOr(&a.ctr->overflow, 16u);
+        break;
+      }
+      a.frags[node + k] = make_uint2(prev[k], order);
+      if (prev[k] == 0xffffffffu)
+        fresh |= bit[k];
+    }
+    node += 4u;
+  }
+  if (!fresh)
+    return;
+  uint32_t t = warp_alloc(&a.ctr->touched_count, (uint32_t)__popc(fresh));
+  for (; fresh; fresh &= fresh - 1u)
+    a.touched[t++] = row + (uint32_t)__ffs((int)fresh) - 1u;
+}
+
 /* One (row, 32-sample chunk) item of a suffix record (nl: records queued):
  * the reference's edge walk from the folded chunk start; covered samples in
  * front of the opaque depth get a fragment. */
@@ -2673,17 +2726,23 @@ __device__ __forceinline__ void oraster_item(const FrameArgs &a, uint32_t it, ui
   float w1 = fold_add(fold_add(r.w0[1], r.dy[1], jr), r.dx[1], kc);
   float w2 = fold_add(fold_add(r.w0[2], r.dy[2], jr), r.dx[2], kc);
   float z = flat ? fold_add(fold_add(r.zc[0], r.zc[2], jr), r.zc[1], kc) : 0.0f;
-  const uint32_t rowbase = (uint32_t)y * (uint32_t)a.width;
-  for (int x = xs; x <= xe; x++) {
+  /* the chunk's covered samples in front of the opaque depth, then nodes for
+   * all of them at once, then their list heads four at a time: the walk, the
+   * allocation and each exchange would otherwise wait for one another at
+   * every sample (66 us against 34, 1280x720 SSAA 2 with 32 blended meshes;
+   * and a chunk's nodes lie together, which the fold reads 50 -> 38 us) */
+  const uint32_t row = (uint32_t)y * (uint32_t)a.width + (uint32_t)xs;
+  uint32_t m = 0;
+#pragma unroll 4
+  for (int i = 0; i <= xe - xs; i++) {
     if (w0 >= 0.0f && w1 >= 0.0f && w2 >= 0.0f) {
       float zz = z;
       if (!flat) {
         const float b0 = w0 * r.inv_area, b1 = w1 * r.inv_area, b2 = w2 * r.inv_area;
         zz = b0 * r.zc[0] + b1 * r.zc[1] + b2 * r.zc[2];
       }
-      const uint32_t px = rowbase + (uint32_t)x;
-      if (a.ordered_keep_all || zz < a.depth[px])
-        push_fragment(a, px, r.order);
+      if (a.ordered_keep_all || zz < __ldg(a.depth + row + i))
+        m |= 1u << i;
     }
     w0 = __fadd_rn(w0, r.dx[0]);
     w1 = __fadd_rn(w1, r.dx[1]);
@@ -2691,6 +2750,9 @@ __device__ __forceinline__ void oraster_item(const FrameArgs &a, uint32_t it, ui
     if (flat)
       z = __fadd_rn(z, r.zc[1]);
   }
+  if (!m)
+    return;
+  push_fragments(a, row, m, r.order);
 }
 
 __device__ __forceinline__ uint32_t olist_len(const FrameArgs &a) {
@@ -3177,17 +3239,21 @@ __device__ __forceinline__ void ofold_item(const FrameArgs &a, uint32_t i) {
   const uint32_t head = a.frag_head[px];
   uint32_t ord[MAX];                      /* order; WIRE: node */
   unsigned long long key[WIRE ? MAX : 1]; /* WIRE: sort keys   */
-  uint32_t cnt = 0, total = 0;
+  uint32_t cnt = 0, total = 0, rest = 0xffffffffu; /* first node past MAX */
   for (uint32_t node = head; node != 0xffffffffu && node < a.frag_cap;) {
     const uint2 f = a.frags[node];
-    if (cnt < MAX) {
-      if (WIRE)
-        key[cnt] = frag_key(a, node, f.y);
+    if (cnt < MAX)
       ord[cnt++] = WIRE ? node : f.y;
-    }
+    else if (total == MAX)
+      rest = node;
     if (++total > a.frag_cap)
       break;
     node = f.x;
+  }
+  if (WIRE && total <= MAX) { /* past the walk, whose loads wait for one another */
+#pragma unroll 4
+    for (uint32_t k = 0; k < cnt; k++)
+      key[WIRE ? k : 0] = frag_key(a, ord[k], a.frags[ord[k]].y);
   }
   const int x = (int)(px % (uint32_t)a.width), y = (int)(px / (uint32_t)a.width);
   OFold st;
@@ -3217,16 +3283,21 @@ __device__ __forceinline__ void ofold_item(const FrameArgs &a, uint32_t i) {
       return;
     }
     ulonglong2 *sc = a.oscratch + base;
-    uint32_t m = 0;
-    for (uint32_t node = head; node != 0xffffffffu && node < a.frag_cap && m < total;) {
+    uint32_t m = cnt;
+#pragma unroll 4
+    for (uint32_t k = 0; k < cnt; k++)
+      sc[k] = WIRE ? make_ulonglong2((unsigned long long)a.frags[ord[k]].y,
+                                     (unsigned long long)ord[k])
+                   : make_ulonglong2((unsigned long long)ord[k], (unsigned long long)ord[k]);
+    for (uint32_t node = rest; node != 0xffffffffu && node < a.frag_cap && m < total;) {
       const uint2 f = a.frags[node];
-      sc[m++] = WIRE ? make_ulonglong2(frag_key(a, node, f.y), (unsigned long long)node)
-                     : make_ulonglong2((unsigned long long)f.y, (unsigned long long)f.y);
+      sc[m++] = make_ulonglong2((unsigned long long)f.y, WIRE ? (unsigned long long)node
+                                                               : (unsigned long long)f.y);
       node = f.x;
     }
-    if (WIRE) { /* left to wlong_item: the list's place and length ride in buffers whose
-                   values for this sample are spent (head, unused hdr component); the
-                   queue takes the shading list's place */
+    if (WIRE) { /* left to wlong_item as (payload, node) pairs: the list's place and length
+                   ride in buffers whose values for this sample are spent (head, unused
+                   hdr component); the queue takes the shading list's place */
       a.frag_head[px] = base;
       a.hdr[px].w = __uint_as_float(m);
       a.shade_list[warp_alloc1(&a.ctr->wlong_count)] = px;
@@ -3265,15 +3336,19 @@ struct WLongSmem {
   uint2 draw[32]; /* flags, object id */
 };
 
-__device__ __forceinline__ void wlong_sort(WLongSmem &sm, ulonglong2 *sc, uint32_t n,
-                                           uint32_t lane) {
+__device__ __forceinline__ void wlong_sort(const FrameArgs &a, WLongSmem &sm, ulonglong2 *sc,
+                                           uint32_t n, uint32_t lane) {
   uint32_t P = 64;
   while (P < n)
     P <<= 1;
   for (uint32_t i = lane; i < P; i += 32u) {
-    const ulonglong2 e = i < n ? sc[i] : make_ulonglong2(~0ull, 0ull);
-    sm.key[i] = e.x;
-    sm.node[i] = (uint32_t)e.y;
+    if (i < n) {
+      const ulonglong2 e = sc[i];
+      sm.key[i] = frag_key(a, (uint32_t)e.y, (uint32_t)e.x);
+      sm.node[i] = (uint32_t)e.y;
+    } else {
+      sm.key[i] = ~0ull;
+    }
   }
   __syncwarp();
   for (uint32_t size = 2; size <= P; size <<= 1)
@@ -3302,10 +3377,15 @@ __device__ __forceinline__ void wlong_item(const FrameArgs &a, uint32_t q, WLong
   ulonglong2 *sc = a.oscratch + a.frag_head[px];
   const int x = (int)(px % (uint32_t)a.width), y = (int)(px / (uint32_t)a.width);
   const bool in_smem = n <= WLONG_SORT;
-  if (in_smem)
-    wlong_sort(sm, sc, n, lane);
-  else if (lane == 0)
-    heapsort_keys(sc, n);
+  if (in_smem) {
+    wlong_sort(a, sm, sc, n, lane);
+  } else {
+    for (uint32_t i = lane; i < n; i += 32u)
+      sc[i].x = frag_key(a, (uint32_t)sc[i].y, (uint32_t)sc[i].x);
+    __syncwarp();
+    if (lane == 0)
+      heapsort_keys(sc, n);
+  }
   __syncwarp();
   OFold st;
   ofold_begin(a, st, px, x, y);
