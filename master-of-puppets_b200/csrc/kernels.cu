@@ -10,8 +10,8 @@
  *   k_raster_*   coverage + depth into a  rasterizer.c:1926-1960 (the
  *                64-bit atomicMin key     incremental edge walk and the
  *                buffer (small records:   strict depth test; replaces the
- *                thread each; large:      single-threaded centroid binning
- *                (row, chunk) items)      of rasterizer_mt.c)
+ *                thread each; large: a    single-threaded centroid binning
+ *                warp's rows or bands)    of rasterizer_mt.c)
  *   k_resolve    background + compaction  rasterizer.c:2785-2792
  *   k_shade      deferred shading + ACES  rasterizer.c:1961-2108, 2776-2803
  *   k_post       FXAA + post + SSAA box   rasterizer.c:2625-2761,
@@ -1204,8 +1204,7 @@ __global__ void k_raster_small(FrameArgs a) {
     raster_small_item(a, base + lane < n, base + lane);
 }
 
-/* Exclusive scan of a record list's item counts (the ordered, wireframe and
- * shadow lists) by one block of 1024:
+/* Exclusive scan of the shadow list's item counts by one block of 1024:
  * tiles of 4096 counts (4 consecutive per thread), warp-shuffle scans, the
  * next tile's counts loaded before the current one is scanned; part holds
  * >= 32 words. */

@@ -9,11 +9,12 @@ cases
   frame        the 1920x1080 SSAA-2 frame of 1,470,464 triangles, 7 lights,
                IBL (k_vertex .. k_post<2>)
   transparent  the same frame with every third instance blended
-               (k_ocount, k_oscan, k_oraster, k_ofold)
+               (k_ocount, k_oraster, k_ofold)
   shadow       the same frame with the directional light casting shadows
                (k_shadow_tri, k_shadow_scan, k_shadow_large, 1024^2 map)
   batch        16 viewports of the same scene in one batched launch
-               (k_batch_prepare, k_b_items, k_b_shade, k_b_post)
+               (k_batch_prepare, k_b_items, k_b_clip, k_b_rsmall,
+               k_b_rlarge, k_b_resolve, k_b_shade, k_b_post)
   small        the 800x600 sphere-and-plane frame
 """
 import argparse
