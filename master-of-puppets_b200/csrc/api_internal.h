@@ -185,6 +185,7 @@ struct MopCudaDevice {
   DevArena irr, pf, brdf;
   int irr_w = 0, irr_h = 0, pf_w = 0, pf_h = 0, pf_levels = 0, brdf_size = 0;
   DevArena env, ibl_tab; /* device precompute: the environment map and host tables */
+  bool ibl_tab_ready = false; /* the tables have arrived (a call that uploaded them ended well) */
   HostArena h_ibl;
   int env_w = 0, env_h = 0;
   cudaEvent_t ibl_t0 = nullptr, ibl_t1 = nullptr;

@@ -496,8 +496,8 @@ __global__ void __launch_bounds__(256) k_ibl_sky(IblDev a) {
                          sky_b * scale + sun_intensity * 0.8f, 1.0f);
 }
 
-/* Uploads the tables, runs the sky (when sky != null) and the three maps on
- * the device stream, and binds the maps as set_ibl does. */
+/* Uploads the tables (the device's first call), runs the sky (when sky != null)
+ * and the three maps on the device stream, and binds the maps as set_ibl does. */
 int run_precompute(MopCudaDevice *d, const float *env_host, int env_w, int env_h,
                    const SkyArgs *sky, float rotation, float intensity) {
   const IblTables L = table_layout();
@@ -508,7 +508,7 @@ int run_precompute(MopCudaDevice *d, const float *env_host, int env_w, int env_h
   if (rc)
     return rc;
   const size_t env_bytes = (size_t)env_w * env_h * 16;
-  rc = 0;
+  rc = d->ibl_tab.ensure(L.total * 4);
   if (env_host)
     rc |= d->h_ibl.ensure(env_bytes);
   rc |= d->env.ensure(env_bytes);
@@ -518,21 +518,16 @@ int run_precompute(MopCudaDevice *d, const float *env_host, int env_w, int env_h
   if (rc)
     return MOPCUDA_ENOMEM;
   cudaStream_t st = d->stream;
-  if (!d->ibl_tab.p) {
-    const std::vector<float> &t = host_tables();
-    if (d->ibl_tab.ensure(L.total * 4))
-      return MOPCUDA_ENOMEM;
-    const cudaError_t e = cudaMemcpy(d->ibl_tab.p, t.data(), L.total * 4, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      d->ibl_tab.release();
-      return fail(MOPCUDA_ECUDA, "ibl tables: %s", cudaGetErrorString(e));
-    }
-  }
   if (!d->ibl_t0) {
     CU_TRY(cudaEventCreate(&d->ibl_t0));
     CU_TRY(cudaEventCreate(&d->ibl_t1));
   }
   CU_TRY(cudaEventRecord(d->ibl_t0, st));
+  /* on the kernels' stream: a blocking copy from pageable memory may return with
+   * its last bytes still on the way, and nothing would order the kernels behind it */
+  if (!d->ibl_tab_ready)
+    CU_TRY(cudaMemcpyAsync(d->ibl_tab.p, host_tables().data(), L.total * 4,
+                           cudaMemcpyHostToDevice, st));
   if (env_host) {
     memcpy(d->h_ibl.p, env_host, env_bytes);
     CU_TRY(cudaMemcpyAsync(d->env.p, d->h_ibl.p, env_bytes, cudaMemcpyHostToDevice, st));
@@ -574,7 +569,10 @@ int run_precompute(MopCudaDevice *d, const float *env_host, int env_w, int env_h
   d->ibl_int = intensity > 0.0f ? intensity : 1.0f;
   d->ibl_on = true;
   /* the staging buffer is reused by the next call: wait for the copies */
-  return mc_bounded_sync(d, d->ibl_t1, FRAME_TIMEOUT_MS);
+  rc = mc_bounded_sync(d, d->ibl_t1, FRAME_TIMEOUT_MS);
+  if (!rc)
+    d->ibl_tab_ready = true;
+  return rc;
 }
 
 } // namespace
