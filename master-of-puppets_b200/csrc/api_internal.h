@@ -241,6 +241,11 @@ struct MopCudaDevice {
 /* Bounded host waits (20 us polls); every device wait of the library. */
 int mc_bounded_sync(MopCudaDevice *d, cudaEvent_t ev, int timeout_ms);
 int mc_stream_sync(MopCudaDevice *d, int timeout_ms);
+/* n bytes to device memory, from the host or the device, there when the call
+ * returns: a blocking copy from pageable memory may return once its source is
+ * staged and one within the device once it is queued, and the streams of the
+ * kernels that read them are non-blocking. */
+cudaError_t mc_upload(void *dst, const void *src, size_t n);
 /* Completes a launched frame (re-running it on overflow) before state it
  * reads changes. */
 int mc_finish_pending(MopCudaDevice *d);

@@ -40,9 +40,9 @@ static int copy_ibl(MopCudaScene *s, const MopCudaDevice *d) {
                bb = (size_t)d->brdf_size * d->brdf_size * 16;
   if (s->irr.ensure(ib) || s->pf.ensure(pb) || s->brdf.ensure(bb))
     return MOPCUDA_ENOMEM;
-  CU_TRY(cudaMemcpy(s->irr.p, d->irr.p, ib, cudaMemcpyDeviceToDevice));
-  CU_TRY(cudaMemcpy(s->pf.p, d->pf.p, pb, cudaMemcpyDeviceToDevice));
-  CU_TRY(cudaMemcpy(s->brdf.p, d->brdf.p, bb, cudaMemcpyDeviceToDevice));
+  CU_TRY(mc_upload(s->irr.p, d->irr.p, ib));
+  CU_TRY(mc_upload(s->pf.p, d->pf.p, pb));
+  CU_TRY(mc_upload(s->brdf.p, d->brdf.p, bb));
   s->irr_w = d->irr_w;
   s->irr_h = d->irr_h;
   s->pf_w = d->pf_w;
@@ -233,11 +233,9 @@ int mc_scene_sync(MopCudaScene *s) {
       s->d_lights.ensure(sizeof(LightRec) * (s->lights.size() + 1)))
     return MOPCUDA_ENOMEM;
   if (nd)
-    CU_TRY(cudaMemcpy(s->d_bounds.p, s->bounds.data(), sizeof(DrawBound) * nd,
-                      cudaMemcpyHostToDevice));
+    CU_TRY(mc_upload(s->d_bounds.p, s->bounds.data(), sizeof(DrawBound) * nd));
   if (!s->lights.empty())
-    CU_TRY(cudaMemcpy(s->d_lights.p, s->lights.data(), sizeof(LightRec) * s->lights.size(),
-                      cudaMemcpyHostToDevice));
+    CU_TRY(mc_upload(s->d_lights.p, s->lights.data(), sizeof(LightRec) * s->lights.size()));
   s->dev_version = s->version;
   return MOPCUDA_OK;
 }

@@ -131,6 +131,13 @@ int mc_bounded_sync(MopCudaDevice *d, cudaEvent_t ev, int timeout_ms) {
   }
 }
 
+cudaError_t mc_upload(void *dst, const void *src, size_t n) {
+  if (!n)
+    return cudaSuccess;
+  const cudaError_t e = cudaMemcpy(dst, src, n, cudaMemcpyDefault);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 int mc_stream_sync(MopCudaDevice *d, int timeout_ms) {
   cudaEvent_t e;
   CU_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -218,7 +225,7 @@ extern "C" MopCudaBuffer *mopcuda_buffer_create(MopCudaDevice *d, const void *da
   }
   if (size) {
     memcpy(b->h, data, size);
-    if (cudaMemcpy(b->d, data, size, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (mc_upload(b->d, data, size) != cudaSuccess) {
       cudaGetLastError();
       cudaFree(b->d);
       free(b->h);
@@ -258,7 +265,7 @@ extern "C" int mopcuda_buffer_update(MopCudaDevice *d, MopCudaBuffer *b, const v
     return rc;
   if (b->h)
     memcpy((uint8_t *)b->h + offset, data, size);
-  CU_TRY(cudaMemcpy((uint8_t *)b->d + offset, data, size, cudaMemcpyHostToDevice));
+  CU_TRY(mc_upload((uint8_t *)b->d + offset, data, size));
   return MOPCUDA_OK;
 }
 
@@ -304,7 +311,7 @@ static MopCudaTexture *tex_create(MopCudaDevice *d, int w, int h, const void *da
     return nullptr;
   }
   memcpy(t->hcopy, data, bytes);
-  if (cudaMemcpy(t->d, data, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (mc_upload(t->d, data, bytes) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(t->d);
     free(t->hcopy);
@@ -480,9 +487,9 @@ extern "C" int mopcuda_set_ibl(MopCudaDevice *d, const float *irr, int iw, int i
   size_t ib = (size_t)iw * ih * 16, pb = pf_px * 16, bb = (size_t)bs * bs * 16;
   if (d->irr.ensure(ib) || d->pf.ensure(pb) || d->brdf.ensure(bb))
     return MOPCUDA_ENOMEM;
-  CU_TRY(cudaMemcpy(d->irr.p, irr, ib, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(d->pf.p, pf, pb, cudaMemcpyHostToDevice));
-  CU_TRY(cudaMemcpy(d->brdf.p, brdf, bb, cudaMemcpyHostToDevice));
+  CU_TRY(mc_upload(d->irr.p, irr, ib));
+  CU_TRY(mc_upload(d->pf.p, pf, pb));
+  CU_TRY(mc_upload(d->brdf.p, brdf, bb));
   d->irr_w = iw;
   d->irr_h = ih;
   d->pf_w = pw;
