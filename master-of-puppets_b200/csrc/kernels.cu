@@ -96,13 +96,17 @@ __device__ __forceinline__ float4 xform(const float *m, float x, float y, float 
   return r;
 }
 
-__device__ __forceinline__ int find_draw_by(const DrawRec *draws, uint32_t n, uint32_t g,
-                                            bool by_vertex) {
-  uint32_t lo = 0, hi = n; /* last draw with base <= g */
+__device__ __forceinline__ uint32_t draw_base(const DrawRec *draws, uint32_t i, bool by_vertex) {
+  return by_vertex ? draws[i].vbase : draws[i].tbase;
+}
+
+/* The last of draws [lo, n) with base <= g (draws[lo] has). */
+__device__ __forceinline__ int find_draw_by(const DrawRec *draws, uint32_t lo, uint32_t n,
+                                            uint32_t g, bool by_vertex) {
+  uint32_t hi = n;
   while (hi - lo > 1) {
-    uint32_t mid = (lo + hi) >> 1;
-    uint32_t b = by_vertex ? draws[mid].vbase : draws[mid].tbase;
-    if (b <= g)
+    const uint32_t mid = (lo + hi) >> 1;
+    if (draw_base(draws, mid, by_vertex) <= g)
       lo = mid;
     else
       hi = mid;
@@ -115,22 +119,26 @@ __device__ __forceinline__ int find_draw_by(const DrawRec *draws, uint32_t n, ui
  * Every vertex and triangle waits for its draw first; a binary search per
  * thread is 8 to 10 loads one after another for 256 to 1,000 draws: the vertices
  * of 2 M triangles in 1,000 draws took 126 instead of 109 us, their setup 88
- * instead of 76, 64 views' setup 895 instead of 745. */
+ * instead of 76, 64 views' setup 895 instead of 745.  A lane that is not there
+ * after FIND_STEPS steps (draws of a few items, or empty ones: each costs a
+ * load) searches the rest: stepping on took 4.4 ms over 20,000 empty draws. */
+#define FIND_STEPS 4
 __device__ __forceinline__ int find_draw_warp(const DrawRec *draws, uint32_t n, uint32_t g0,
                                               uint32_t g, bool by_vertex) {
   uint32_t lo = 0, hi = n;
   while (hi - lo > 1) {
     const uint32_t step = (hi - lo + 31u) >> 5;
     const uint32_t cand = lo + (threadIdx.x & 31u) * step;
-    bool le = false;
-    if (cand < hi)
-      le = (by_vertex ? draws[cand].vbase : draws[cand].tbase) <= g0;
-    const uint32_t pass = __ballot_sync(0xffffffffu, le);
+    const uint32_t pass =
+        __ballot_sync(0xffffffffu, cand < hi && draw_base(draws, cand, by_vertex) <= g0);
     lo += (uint32_t)(31 - __clz((int)pass)) * step;
     hi = min(hi, lo + step);
   }
-  while (lo + 1u < n && (by_vertex ? draws[lo + 1u].vbase : draws[lo + 1u].tbase) <= g)
+  for (int k = 1; lo + 1u < n && draw_base(draws, lo + 1u, by_vertex) <= g; k++) {
     lo++;
+    if (k == FIND_STEPS)
+      return find_draw_by(draws, lo, n, g, by_vertex);
+  }
   return (int)lo;
 }
 
@@ -1025,7 +1033,7 @@ template <bool SH>
 __device__ __forceinline__ void clip_item(const FrameArgs &a, uint32_t qi) {
   {
     uint32_t t = a.clipq[qi];
-    const DrawRec &d = a.draws[find_draw_by(a.draws, a.draw_count, t, false)];
+    const DrawRec &d = a.draws[find_draw_by(a.draws, 0u, a.draw_count, t, false)];
     uint32_t lt = t - d.tbase;
     CV buf0[MAX_CLIP], buf1[MAX_CLIP];
     for (int k = 0; k < 3; k++)
