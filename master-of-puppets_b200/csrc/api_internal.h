@@ -146,6 +146,8 @@ struct MopCudaDevice {
   int num_sms = 148;
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr; /* asynchronous readbacks */
+  cudaStream_t up_stream = nullptr;   /* uploads (mc_upload), beside a running frame */
+  cudaEvent_t up_ev = nullptr;        /* after the last upload */
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t pick_ev = nullptr; /* the allocation-free pick's bounded wait */
   cudaEvent_t stage_ev[MOPCUDA_STAGES + 1] = {};
@@ -241,11 +243,12 @@ struct MopCudaDevice {
 /* Bounded host waits (20 us polls); every device wait of the library. */
 int mc_bounded_sync(MopCudaDevice *d, cudaEvent_t ev, int timeout_ms);
 int mc_stream_sync(MopCudaDevice *d, int timeout_ms);
-/* n bytes to device memory, from the host or the device, there when the call
- * returns: a blocking copy from pageable memory may return once its source is
- * staged and one within the device once it is queued, and the streams of the
+/* n bytes to device memory, from the host (copied or staged when the call
+ * returns) or the device, ahead of all later work of d->stream; a launch core's
+ * stream waits for d->up_ev.  On the legacy stream nothing would be ordered
+ * behind a copy whose last bytes are still on the way: the streams of the
  * kernels that read them are non-blocking. */
-cudaError_t mc_upload(void *dst, const void *src, size_t n);
+cudaError_t mc_upload(MopCudaDevice *d, void *dst, const void *src, size_t n);
 /* Completes a launched frame (re-running it on overflow) before state it
  * reads changes. */
 int mc_finish_pending(MopCudaDevice *d);

@@ -27,7 +27,7 @@
 /* ------------------------------------------------------------------------
  * scene
  * ------------------------------------------------------------------------ */
-static int copy_ibl(MopCudaScene *s, const MopCudaDevice *d) {
+static int copy_ibl(MopCudaScene *s, MopCudaDevice *d) {
   s->ibl_on = d->ibl_on;
   if (!d->ibl_on)
     return MOPCUDA_OK;
@@ -40,9 +40,9 @@ static int copy_ibl(MopCudaScene *s, const MopCudaDevice *d) {
                bb = (size_t)d->brdf_size * d->brdf_size * 16;
   if (s->irr.ensure(ib) || s->pf.ensure(pb) || s->brdf.ensure(bb))
     return MOPCUDA_ENOMEM;
-  CU_TRY(mc_upload(s->irr.p, d->irr.p, ib));
-  CU_TRY(mc_upload(s->pf.p, d->pf.p, pb));
-  CU_TRY(mc_upload(s->brdf.p, d->brdf.p, bb));
+  CU_TRY(mc_upload(d, s->irr.p, d->irr.p, ib));
+  CU_TRY(mc_upload(d, s->pf.p, d->pf.p, pb));
+  CU_TRY(mc_upload(d, s->brdf.p, d->brdf.p, bb));
   s->irr_w = d->irr_w;
   s->irr_h = d->irr_h;
   s->pf_w = d->pf_w;
@@ -233,9 +233,10 @@ int mc_scene_sync(MopCudaScene *s) {
       s->d_lights.ensure(sizeof(LightRec) * (s->lights.size() + 1)))
     return MOPCUDA_ENOMEM;
   if (nd)
-    CU_TRY(mc_upload(s->d_bounds.p, s->bounds.data(), sizeof(DrawBound) * nd));
+    CU_TRY(mc_upload(s->dev, s->d_bounds.p, s->bounds.data(), sizeof(DrawBound) * nd));
   if (!s->lights.empty())
-    CU_TRY(mc_upload(s->d_lights.p, s->lights.data(), sizeof(LightRec) * s->lights.size()));
+    CU_TRY(mc_upload(s->dev, s->d_lights.p, s->lights.data(),
+                     sizeof(LightRec) * s->lights.size()));
   s->dev_version = s->version;
   return MOPCUDA_OK;
 }
@@ -632,6 +633,7 @@ int LaunchCore::stage() {
     if ((rc = stage_shadow(k, hd + scene_draw_off[k], d)))
       return rc;
   }
+  CU_TRY(cudaStreamWaitEvent(stream, dev->up_ev, 0)); /* what the kernels read is there */
   any_shadow = false;
   for (size_t k = 0; k < scenes.size(); k++)
     any_shadow |= shadows[k].size > 0;

@@ -95,6 +95,8 @@ extern "C" MopCudaDevice *mopcuda_device_create(int ordinal) {
   d->cfg.num_sms = d->num_sms;
   if (cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&d->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&d->up_stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&d->up_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&d->ev0) != cudaSuccess || cudaEventCreate(&d->ev1) != cudaSuccess ||
       cudaEventCreateWithFlags(&d->pick_ev, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
@@ -131,11 +133,13 @@ int mc_bounded_sync(MopCudaDevice *d, cudaEvent_t ev, int timeout_ms) {
   }
 }
 
-cudaError_t mc_upload(void *dst, const void *src, size_t n) {
+cudaError_t mc_upload(MopCudaDevice *d, void *dst, const void *src, size_t n) {
   if (!n)
     return cudaSuccess;
-  const cudaError_t e = cudaMemcpy(dst, src, n, cudaMemcpyDefault);
-  return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+  cudaError_t e = cudaMemcpyAsync(dst, src, n, cudaMemcpyDefault, d->up_stream);
+  if (e == cudaSuccess)
+    e = cudaEventRecord(d->up_ev, d->up_stream);
+  return e == cudaSuccess ? cudaStreamWaitEvent(d->stream, d->up_ev, 0) : e;
 }
 
 int mc_stream_sync(MopCudaDevice *d, int timeout_ms) {
@@ -196,6 +200,9 @@ extern "C" void mopcuda_device_destroy(MopCudaDevice *d) {
       cudaEventDestroy(d->stage_ev[i]);
   cudaStreamSynchronize(d->copy_stream);
   cudaStreamDestroy(d->copy_stream);
+  cudaStreamSynchronize(d->up_stream);
+  cudaStreamDestroy(d->up_stream);
+  cudaEventDestroy(d->up_ev);
   cudaStreamDestroy(d->stream);
   delete d;
 }
@@ -225,7 +232,7 @@ extern "C" MopCudaBuffer *mopcuda_buffer_create(MopCudaDevice *d, const void *da
   }
   if (size) {
     memcpy(b->h, data, size);
-    if (mc_upload(b->d, data, size) != cudaSuccess) {
+    if (mc_upload(d, b->d, data, size) != cudaSuccess) {
       cudaGetLastError();
       cudaFree(b->d);
       free(b->h);
@@ -265,7 +272,7 @@ extern "C" int mopcuda_buffer_update(MopCudaDevice *d, MopCudaBuffer *b, const v
     return rc;
   if (b->h)
     memcpy((uint8_t *)b->h + offset, data, size);
-  CU_TRY(mc_upload((uint8_t *)b->d + offset, data, size));
+  CU_TRY(mc_upload(d, (uint8_t *)b->d + offset, data, size));
   return MOPCUDA_OK;
 }
 
@@ -311,7 +318,7 @@ static MopCudaTexture *tex_create(MopCudaDevice *d, int w, int h, const void *da
     return nullptr;
   }
   memcpy(t->hcopy, data, bytes);
-  if (mc_upload(t->d, data, bytes) != cudaSuccess) {
+  if (mc_upload(d, t->d, data, bytes) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(t->d);
     free(t->hcopy);
@@ -487,9 +494,9 @@ extern "C" int mopcuda_set_ibl(MopCudaDevice *d, const float *irr, int iw, int i
   size_t ib = (size_t)iw * ih * 16, pb = pf_px * 16, bb = (size_t)bs * bs * 16;
   if (d->irr.ensure(ib) || d->pf.ensure(pb) || d->brdf.ensure(bb))
     return MOPCUDA_ENOMEM;
-  CU_TRY(mc_upload(d->irr.p, irr, ib));
-  CU_TRY(mc_upload(d->pf.p, pf, pb));
-  CU_TRY(mc_upload(d->brdf.p, brdf, bb));
+  CU_TRY(mc_upload(d, d->irr.p, irr, ib));
+  CU_TRY(mc_upload(d, d->pf.p, pf, pb));
+  CU_TRY(mc_upload(d, d->brdf.p, brdf, bb));
   d->irr_w = iw;
   d->irr_h = ih;
   d->pf_w = pw;
