@@ -276,15 +276,19 @@ void mc_pool_need(uint64_t T, uint64_t V, uint32_t fan_num, uint32_t large_num,
 uint64_t mc_view_bytes(const MopCudaScene *s, uint64_t samples, uint64_t pixels) {
   unsigned long long need[4];
   mc_pool_need(s->tris, s->verts, 1, 1, need);
-  const uint64_t pools = 64ull * need[0] + (sizeof(RasterRec) + sizeof(ShadeRec)) * need[1] +
-                         4ull * need[2] + 8ull * need[3];
-  /* an ordered suffix: hdr, list heads and touched samples, a fragment per
-   * sample and the suffix-record list */
-  const uint64_t suffix =
-      s->ordered_tris ? 32ull * samples + (s->wire ? 16ull : 8ull) * (s->ordered_tris + need[2]) +
-                            4096ull * 8ull
-                      : 0ull;
-  return 28ull * samples + 4ull * pixels + pools / 2 + suffix +
+  /* size_pools: four vertex streams; a record, its shading record and chunk
+   * offset; the clip queue; two lists with their item offsets */
+  const uint64_t pools = 64ull * need[0] + (sizeof(RasterRec) + sizeof(ShadeRec) + 4ull) * need[1] +
+                         4ull * need[2] + 16ull * need[3];
+  /* stage_suffix: hdr, list head and touched sample per sample, a fragment per
+   * sample with its sort scratch (and its line plot), the record lists */
+  uint64_t suffix = 0;
+  if (s->ordered_tris)
+    suffix = 24ull * samples + (24ull + (s->wire ? sizeof(WirePlot) : 0ull)) * (samples + 4096ull) +
+             (s->wire ? 16ull : 8ull) * (s->ordered_tris + need[2]);
+  /* set_layout: key, shading list entry, half a chunk start, pre, out, depth
+   * and ID per sample */
+  return 36ull * samples + 4ull * pixels + pools / 2 + suffix +
          sizeof(DrawRec) * s->draws.size();
 }
 
