@@ -699,10 +699,7 @@ int LaunchCore::stage_suffix() {
     rc |= olist.ensure(4ull * ol);
     rc |= olist_items.ensure(4ull * ol);
   }
-  if (frag_pool < fr) {
-    rc |= frags.ensure(8ull * fr);
-    rc |= oscratch.ensure(16ull * fr);
-  }
+  rc |= size_fragments(fr);
   if (any_wire && wlist_pool < wl) {
     rc |= wlist.ensure(4ull * wl);
     rc |= wlist_items.ensure(4ull * wl);
@@ -710,14 +707,23 @@ int LaunchCore::stage_suffix() {
   if (rc)
     return MOPCUDA_ENOMEM;
   olist_pool = std::min(olist.cap / 4, olist_items.cap / 4);
-  frag_pool = std::min(frags.cap / 8, oscratch.cap / 16);
   wlist_pool = std::min(wlist.cap / 4, wlist_items.cap / 4);
-  if (any_wire && wplots.ensure(sizeof(WirePlot) * frag_pool))
-    return MOPCUDA_ENOMEM;
   void *after_[10] = {hdr.p, frag_head.p, touched.p, frags.p, olist.p, olist_items.p,
                       wlist.p, wlist_items.p, wplots.p, oscratch.p};
   if (memcmp(before, after_, sizeof before) != 0)
     suffix_moved = true;
+  return MOPCUDA_OK;
+}
+
+/* Room for fr fragments: nodes, sort scratch and, in a launch with wireframe
+ * draws, a line plot beside each node. */
+int LaunchCore::size_fragments(unsigned long long fr) {
+  if (frags.ensure(8ull * fr) || oscratch.ensure(16ull * fr) ||
+      (any_wire && wplots.ensure(sizeof(WirePlot) * fr)))
+    return MOPCUDA_ENOMEM;
+  frag_pool = std::min(frags.cap / 8, oscratch.cap / 16);
+  if (any_wire)
+    frag_pool = std::min<unsigned long long>(frag_pool, wplots.cap / sizeof(WirePlot));
   return MOPCUDA_OK;
 }
 
@@ -918,13 +924,8 @@ int LaunchCore::after(bool *rerun, int attempt) {
       rc |= olist_items.ensure(4ull * ol);
       olist_pool = std::min(olist.cap / 4, olist_items.cap / 4);
     }
-    if ((st->overflow & 32u) && fr > frag_pool) {
-      rc |= frags.ensure(8ull * fr);
-      rc |= oscratch.ensure(16ull * fr);
-      frag_pool = std::min(frags.cap / 8, oscratch.cap / 16);
-    }
-    if (any_wire)
-      rc |= wplots.ensure(sizeof(WirePlot) * frag_pool);
+    if ((st->overflow & 32u) && fr > frag_pool)
+      rc |= size_fragments(fr);
     if (rc)
       return MOPCUDA_ENOMEM;
   }

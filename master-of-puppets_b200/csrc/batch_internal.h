@@ -117,6 +117,7 @@ struct LaunchCore {
   void release();
   int stage_shadow(size_t k, const DrawRec *dr, SceneDesc &d);
   int stage_suffix();
+  int size_fragments(unsigned long long fr);
   /* views[i] renders scene scene_of[i] (index into sc); no_color[i] (may be
    * null) marks visibility-only viewports. */
   int set_layout(const MopCudaView *views, const uint32_t *scene_of, const uint8_t *no_color,

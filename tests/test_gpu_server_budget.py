@@ -43,7 +43,7 @@ def _scene(kind):
     return dataclasses.replace(sc, wireframe=kind == "wireframe")
 
 
-@pytest.mark.parametrize("kind", ["plain", "triangles", "blended"])
+@pytest.mark.parametrize("kind", ["plain", "triangles", "blended", "wireframe"])
 def test_estimate_is_what_a_slot_holds(cuda_device, kind):
     sc = _hidden(_scene(kind))
     rs = mopcuda.ResidentScene(cuda_device, sc)
