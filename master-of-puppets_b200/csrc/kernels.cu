@@ -851,13 +851,16 @@ __device__ __forceinline__ uint32_t rec_chunks(const RasterRec &r) {
  * whose group sum goes to *extra_count when given.  (An atomic per record: the
  * setup of 20 views with many large records took 155 us, with the chunk
  * table's counter 290; with the group's shared ones 90.)  An item total past
- * 2^32 carries into the count: flagged (bit 9), the frame fails. */
+ * 2^32 carries into the count, which skips a slot: past `limit` the frame is
+ * flagged (bit 9) and fails, and no list of it is walked (list_items). */
+#define LIST_MAX_ITEMS 0xfff80000u /* a grid's step from 2^32: the walks' indices do not wrap */
+#define WIDE_MAX_ITEMS 0x80000000u /* large_units adds the rows' warps to the bands */
 struct ListPlace {
   uint32_t slot, off;
   unsigned long long extra;
 };
 __device__ __forceinline__ ListPlace push_items(const FrameArgs &a, uint32_t *pair, uint32_t n,
-                                                uint32_t extra,
+                                                uint32_t limit, uint32_t extra,
                                                 unsigned long long *extra_count) {
   const uint32_t mask = __activemask(), lane = threadIdx.x & 31u;
   const uint32_t peers = __match_any_sync(mask, (unsigned long long)(uintptr_t)pair);
@@ -884,13 +887,20 @@ __device__ __forceinline__ ListPlace push_items(const FrameArgs &a, uint32_t *pa
   old = __shfl_sync(peers, old, leader);
   if (extra_count)
     e = __shfl_sync(peers, e, leader);
-  if ((uint32_t)old + sum_n < sum_n)
+  const uint32_t total = (uint32_t)old + sum_n;
+  if (total < sum_n || total > limit)
     atomicOr(&a.ctr->overflow, 512u);
   ListPlace p;
   p.slot = (uint32_t)(old >> 32) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
   p.off = (uint32_t)old + before_n;
   p.extra = e + before_e;
   return p;
+}
+
+/* Items of a record list whose pushes have ended: none when a list of the frame
+ * outgrew its numbering (a skipped slot holds what an earlier frame left there). */
+__device__ __forceinline__ uint32_t list_items(const FrameArgs &a, uint32_t items) {
+  return (a.ctr->overflow & 512u) ? 0u : items;
 }
 
 /* Queues a large record and takes its chunk_w entries (past the capacity it
@@ -902,7 +912,8 @@ __device__ __forceinline__ void push_large(const FrameArgs &a, uint32_t rid, con
                                 ((chunks + BAND_CHUNKS - 1u) / BAND_CHUNKS)
                           : h;
   const ListPlace p = push_items(a, wide ? &a.ctr->wide_items : &a.ctr->large_items, n,
-                                 h * chunks, &a.ctr->chunk_count);
+                                 wide ? WIDE_MAX_ITEMS : LIST_MAX_ITEMS, h * chunks,
+                                 &a.ctr->chunk_count);
   a.large_off[rid] = p.extra + h * chunks <= a.chunk_cap ? (uint32_t)p.extra : 0xffffffffu;
   if (p.slot < a.large_cap) {
     (wide ? a.wide_list : a.large_list)[p.slot] = rid;
@@ -1525,7 +1536,7 @@ __device__ __forceinline__ void wide_band(const FrameArgs &a, uint32_t it, Large
 /* Work of the warps: the bands, then the rows 32 at a time. */
 __device__ __forceinline__ uint32_t large_units(const FrameArgs &a) {
   const uint32_t rows = a.ctr->large_items;
-  return a.ctr->wide_items + rows / 32u + (rows % 32u ? 1u : 0u);
+  return list_items(a, a.ctr->wide_items + rows / 32u + (rows % 32u ? 1u : 0u));
 }
 
 __device__ __forceinline__ void large_unit(const FrameArgs &a, uint32_t u, LargeSmem &q,
@@ -2665,7 +2676,8 @@ __device__ __forceinline__ void ocount_item(const FrameArgs &a, uint32_t i) {
   const RasterRec r = a.rrec[rid];
   if (!rec_live(r, a.width, a.height) || !rec_ordered(a, r))
     return;
-  const ListPlace p = push_items(a, &a.ctr->olist_items, rec_items(r), 0u, nullptr);
+  const ListPlace p = push_items(a, &a.ctr->olist_items, rec_items(r), LIST_MAX_ITEMS,
+                                 0u, nullptr);
   if (p.slot < a.olist_cap) {
     a.olist[p.slot] = rid;
     a.olist_items[p.slot] = p.off;
@@ -2801,7 +2813,7 @@ __device__ __forceinline__ uint32_t olist_len(const FrameArgs &a) {
 __global__ void __launch_bounds__(256) k_oraster(FrameArgs a) {
   pdl_wait();
   const uint32_t nl = olist_len(a);
-  const uint32_t total = a.ctr->olist_items;
+  const uint32_t total = list_items(a, a.ctr->olist_items);
   for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < total;
        it += gridDim.x * blockDim.x)
     oraster_item(a, it, nl);
@@ -2961,7 +2973,7 @@ __device__ __forceinline__ void wcount_item(const FrameArgs &a, uint32_t i) {
     wu_edge(r, e, L);
     n += wu_plots(L);
   }
-  const ListPlace p = push_items(a, &a.ctr->wire_items, n, 0u, nullptr);
+  const ListPlace p = push_items(a, &a.ctr->wire_items, n, LIST_MAX_ITEMS, 0u, nullptr);
   if (p.slot < a.wlist_cap) {
     a.wlist[p.slot] = rid;
     a.wlist_items[p.slot] = p.off;
@@ -3018,7 +3030,7 @@ __device__ __forceinline__ void wplot_item(const FrameArgs &a, uint32_t it) {
 
 __global__ void __launch_bounds__(256) k_wplot(FrameArgs a) {
   pdl_wait();
-  const uint32_t total = a.ctr->wire_items;
+  const uint32_t total = list_items(a, a.ctr->wire_items);
   for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < total;
        it += gridDim.x * blockDim.x)
     wplot_item(a, it);
@@ -3897,13 +3909,13 @@ template <int ST> __device__ __forceinline__ uint32_t stage_count(const FrameArg
   case ST_OCOUNT:
     return a.hdr && a.total_tris ? ordered_record_items(a) : 0u;
   case ST_ORASTER:
-    return a.hdr ? a.ctr->olist_items : 0u;
+    return a.hdr ? list_items(a, a.ctr->olist_items) : 0u;
   case ST_OFOLD:
     return a.hdr ? a.ctr->touched_count : 0u;
   case ST_WCOUNT:
     return a.hdr && a.wire && a.total_tris ? ordered_record_items(a) : 0u;
   case ST_WPLOT:
-    return a.hdr && a.wire ? a.ctr->wire_items : 0u;
+    return a.hdr && a.wire ? list_items(a, a.ctr->wire_items) : 0u;
   case ST_WLONG:
     return a.hdr ? a.ctr->wlong_count : 0u;
   default: /* ST_RESOLVE: chunks of 256 x RESOLVE_PER_THREAD samples */
