@@ -243,6 +243,8 @@ struct MopCudaDevice {
 /* Bounded host waits (20 us polls); every device wait of the library. */
 int mc_bounded_sync(MopCudaDevice *d, cudaEvent_t ev, int timeout_ms);
 int mc_stream_sync(MopCudaDevice *d, int timeout_ms);
+/* What overflow bit 9 of the counters means: any of the numbered lists. */
+const char *mc_items_text();
 /* n bytes to device memory, from the host (copied or staged when the call
  * returns) or the device, ahead of all later work of d->stream; a launch core's
  * stream waits for d->up_ev.  On the legacy stream nothing would be ordered

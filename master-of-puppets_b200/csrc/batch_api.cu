@@ -862,8 +862,7 @@ int LaunchCore::after(bool *rerun, int attempt) {
   if (!st->overflow && !view_over)
     return MOPCUDA_OK;
   if (view_over & 512u)
-    return fail(MOPCUDA_EUNSUPPORTED,
-                "launch: a viewport's large-triangle raster items exceed 2^32");
+    return fail(MOPCUDA_EUNSUPPORTED, "launch: in a viewport, %s", mc_items_text());
   if (attempt >= 8)
     return fail(MOPCUDA_ENOMEM, "launch pools overflowed repeatedly (flags %u/%u)", st->overflow,
                 view_over);

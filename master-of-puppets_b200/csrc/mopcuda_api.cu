@@ -1303,6 +1303,11 @@ extern "C" int mopcuda_frame_io_bytes(MopCudaDevice *d, uint64_t *h2d, uint64_t 
 }
 
 
+const char *mc_items_text() {
+  return "the large triangles' rows, the blended suffix's items or the wireframe's line plots "
+         "exceed 2^32";
+}
+
 /* Waits for the launched frame; re-runs it with larger arenas if any
  * capacity overflowed (the counters say by how much). */
 static int finish_frame(MopCudaDevice *d, int timeout_ms, bool defer_readback) {
@@ -1334,8 +1339,7 @@ static int finish_frame(MopCudaDevice *d, int timeout_ms, bool defer_readback) {
       break;
     }
     if (c->overflow & 512u)
-      return fail(MOPCUDA_EUNSUPPORTED,
-                  "frame: the large triangles' raster items exceed 2^32 in one frame");
+      return fail(MOPCUDA_EUNSUPPORTED, "frame: %s", mc_items_text());
     if (attempt >= 4)
       return fail(MOPCUDA_ENOMEM, "frame arenas overflowed repeatedly (flags %u)", c->overflow);
     d->rec_hint = c->rec_count + c->rec_count / 4 + 1024;
