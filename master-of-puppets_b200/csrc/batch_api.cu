@@ -493,8 +493,7 @@ int LaunchCore::set_layout(const MopCudaView *views, const uint32_t *scene_of,
       continue; /* visibility only: no post effects */
     const int k = r.ssaa - 1;
     lists[(size_t)k * n + post_count[k]++] = i;
-    const uint32_t pw = (uint32_t)(r.width / r.ssaa), ph = (uint32_t)(r.height / r.ssaa);
-    post_tiles[k] += ((pw + 31u) / 32u) * ((ph + 7u) / 8u);
+    post_tiles[k] += post_tile_count(r.width, r.height, r.ssaa);
   }
   CU_TRY(cudaMemcpyAsync(d_posts.p, posts.data(), sizeof(PostArgs) * n, cudaMemcpyHostToDevice,
                          stream));

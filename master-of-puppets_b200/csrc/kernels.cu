@@ -1941,14 +1941,6 @@ __global__ void __launch_bounds__(256, 4) k_shade(FrameArgs a) {
  * a one-sample halo (and each sample's luma) in shared memory with
  * coalesced loads, then each thread filters its ssaa x ssaa samples.
  * ------------------------------------------------------------------------ */
-#define POST_BX 32
-#define POST_BY 8
-/* Presented pixels a thread filters, one above the other: with one at SSAA 1
- * the tile's copies, halo and barriers outweighed its 256 samples. */
-template <int SF> struct PostRows {
-  static constexpr int value = SF == 1 ? 4 : 1; /* 20 views' post 290 -> 184 us */
-};
-
 __device__ __forceinline__ float luma(uchar4 p) {
   return 0.299f * (float)p.x + 0.587f * (float)p.y + 0.114f * (float)p.z;
 }
@@ -1995,7 +1987,7 @@ __device__ __forceinline__ uchar4 fxaa_blend(const uchar4 (*tc)[TW], const float
  * asynchronous copies while the current one is filtered. */
 template <int SF> struct PostSmem {
   static constexpr int OX = 4; /* tile column of the block's first own sample */
-  static constexpr int ROWS = POST_BY * PostRows<SF>::value; /* pixel rows of a tile */
+  static constexpr int ROWS = POST_BY * post_rows(SF); /* pixel rows of a tile */
   static constexpr int TW = POST_BX * SF + 2 * OX, TH = ROWS * SF + 2;
   static constexpr int NBUF = SF <= 3 ? 2 : 1; /* within 48 KB of static shared memory */
   alignas(16) uchar4 c[NBUF][TH][TW];
@@ -2208,14 +2200,13 @@ __device__ __forceinline__ void post_filter(const PostArgs &a, bool vec, PostSme
   __syncthreads();
   const int pw = a.width / SF, ph = a.height / SF;
   const int px = bx * POST_BX + (int)threadIdx.x;
-  const int py = by * PostSmem<SF>::ROWS + (int)threadIdx.y * PostRows<SF>::value;
+  const int py = by * PostSmem<SF>::ROWS + (int)threadIdx.y * post_rows(SF);
   if (px < pw && py < ph)
     post_pixel<SF, TW, FOG>(a, sm.c[buf], sm.l, sm.lut, sm.lut8, sm.thr, px, py);
   __syncthreads();
 }
 
-/* One tile of POST_BX x POST_BY presented pixels (bx, by), copied and
- * filtered with nothing in flight around it. */
+/* One tile (bx, by), copied and filtered with nothing in flight around it. */
 template <int SF, bool FOG>
 __device__ __forceinline__ void post_tile(const PostArgs &a, PostSmem<SF> &sm, int bx, int by) {
   const bool vec = post_vec(a);
@@ -2224,7 +2215,7 @@ __device__ __forceinline__ void post_tile(const PostArgs &a, PostSmem<SF> &sm, i
   post_filter<SF, FOG>(a, vec, sm, 0, bx, by);
 }
 
-/* The thread's samples (PostRows pixels of SF x SF): for SF 1 and 2 their
+/* The thread's samples (post_rows(SF) pixels of SF x SF): for SF 1 and 2 their
  * lumas and the ring around them (without its corners) and their colours are
  * read once, two columns at a time for SF 2 (a thread's samples lie SF words
  * apart, so single words would collide in the banks); most samples end at the
@@ -2236,7 +2227,7 @@ __device__ __forceinline__ void post_pixel(const PostArgs &a, const uchar4 (*s_c
                                            const float (*s_l)[TW], const float *s_lut,
                                            const uint8_t *s_lut8, const float *s_thr, int px,
                                            int py) {
-  constexpr int RP = PostRows<SF>::value, N = SF * RP; /* sample rows */
+  constexpr int RP = post_rows(SF), N = SF * RP; /* sample rows */
   constexpr bool WIN = SF <= 2;
   const int w = a.width, h = a.height, pw = w / SF, ph = h / SF;
   const bool fx = (a.effects & 16u) && w >= 3 && h >= 3;
@@ -2569,9 +2560,7 @@ int mopcuda_launch_frame(const FrameArgs &a, const PostArgs &p, const LaunchCfg 
     cudaStreamWaitEvent(s, post_wait, 0);
   const int sf = p.ssaa;
   dim3 pb(POST_BX, POST_BY);
-  const uint32_t tiles = blocks_for((uint32_t)(p.width / sf), POST_BX) *
-                         blocks_for((uint32_t)(p.height / sf),
-                                    POST_BY * (sf == 1 ? PostRows<1>::value : 1));
+  const uint32_t tiles = post_tile_count(p.width, p.height, sf);
   auto pgrid = [&](int resident) {
     const uint32_t g = (uint32_t)cfg.num_sms * (uint32_t)resident;
     return tiles < g ? (tiles ? tiles : 1u) : g;
@@ -4146,12 +4135,6 @@ __global__ void __launch_bounds__(32 * WLONG_WARPS) k_b_wlong(const FrameArgs *_
   }
 }
 
-template <int SF>
-__device__ __forceinline__ uint32_t post_tiles_of(const PostArgs &p) {
-  const uint32_t pw = (uint32_t)(p.width / SF), ph = (uint32_t)(p.height / SF);
-  return ((pw + POST_BX - 1u) / POST_BX) * ((ph + PostSmem<SF>::ROWS - 1u) / PostSmem<SF>::ROWS);
-}
-
 /* Post tiles of the viewports listed in views (all with ssaa SF). */
 template <int SF, bool FOG>
 __global__ void __launch_bounds__(POST_BX *POST_BY, 4) k_b_post(const PostArgs *__restrict__ posts,
@@ -4164,7 +4147,11 @@ __global__ void __launch_bounds__(POST_BX *POST_BY, 4) k_b_post(const PostArgs *
     uint32_t run = 0;
     for (uint32_t base = 0; base < n; base += 32u) {
       const uint32_t k = base + tid;
-      const uint32_t c = k < n ? post_tiles_of<SF>(posts[views[k]]) : 0u;
+      uint32_t c = 0;
+      if (k < n) {
+        const PostArgs &p = posts[views[k]];
+        c = post_tile_count(p.width, p.height, SF);
+      }
       uint32_t incl = c;
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
