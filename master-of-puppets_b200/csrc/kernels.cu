@@ -468,18 +468,6 @@ __device__ __forceinline__ void ibl_bilinear(const float *d, int w, int h, float
   }
 }
 
-/* x / c for a compile-time c, by Markstein's final step (P. Markstein, IBM J.
- * Res. Dev. 34(1), 1990): q = x * RN(1/c) corrected by its exact remainder
- * rounds correctly when neither underflows.  For the two divisors here the
- * sum with 0.5 that follows equals the division's for every float x below
- * 1e30 (checked exhaustively), tiny quotients being absorbed; 3 instructions
- * instead of a division's dozen. */
-__device__ __forceinline__ float div_const(float x, float c) {
-  const float rc = 1.0f / c; /* folded by the compiler */
-  const float q = x * rc;
-  return __fmaf_rn(__fmaf_rn(-q, c, x), rc, q);
-}
-
 /* dir_to_uv, rasterizer.c:216-222.  atan2f/asinf are CUDA's; glibc's differ
  * in the last ulp for some inputs, which perturbs IBL colour by at most a
  * rounding step. */
