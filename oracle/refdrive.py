@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import unittest
 from pathlib import Path
 
 import numpy as np
@@ -95,11 +96,16 @@ def available() -> bool:
     return REF_SO.exists()
 
 
+class ReferenceMissing(unittest.SkipTest, FileNotFoundError):
+    """The reference library is not built on this machine: a test that compares with it live has
+    nothing to compare with, and is skipped."""
+
+
 def lib(kind: str = "cpu"):
     so = REF_SO if kind == "cpu" else REF_CUDA_SO
     if kind not in _libs:
         if not so.exists():
-            raise FileNotFoundError(f"reference library not built: {so}")
+            raise ReferenceMissing(f"reference library not built: {so}")
         _lib = _libs[kind] = C.CDLL(str(so))
         _lib.refh_create.restype = C.c_void_p
         _lib.refh_create.argtypes = [C.POINTER(RefScene)]
