@@ -338,10 +338,11 @@ void LaunchCore::release() {
   if (stream)
     sync(10000);
   DevArena *arenas[] = {&d_views, &d_frames, &d_view_draws, &d_ctr, &d_status, &d_posts,
-                        &d_post_views, &d_draws, &d_scenes, &clip, &world, &normal, &color,
-                        &rrec, &srec, &clipq, &large_list, &large_items, &wide_list, &wide_items, &large_off, &chunk_w, &keys, &shade_list,
-                        &pre, &out, &depth, &ids, &presented, &hdr, &frag_head, &touched,
-                        &frags, &olist, &olist_items, &wlist, &wlist_items, &wplots, &oscratch};
+                        &d_post_views, &d_draws, &d_scenes, &clip, &world, &normal, &color, &rrec,
+                        &srec, &clipq, &large_list, &large_items, &wide_list, &wide_items,
+                        &large_off, &chunk_w, &keys, &shade_list, &pre, &out, &depth, &ids,
+                        &presented, &hdr, &frag_head, &touched, &frags, &olist, &olist_items,
+                        &wlist, &wlist_items, &wplots, &oscratch};
   for (DevArena *a : arenas)
     a->release();
   frag_pool = olist_pool = wlist_pool = 0;
@@ -369,11 +370,11 @@ void LaunchCore::release() {
 void LaunchCore::trim() {
   if (stream)
     sync(10000);
-  DevArena *arenas[] = {&clip,       &world, &normal,  &color,      &rrec,      &srec,
-                        &clipq,      &large_list, &large_items, &wide_list, &wide_items, &large_off, &chunk_w, &keys, &shade_list, &pre,
-                        &out,        &depth, &ids,     &presented,  &hdr,       &frag_head,
-                        &touched,    &frags, &olist,   &olist_items, &wlist, &wlist_items,
-                        &wplots,     &oscratch};
+  DevArena *arenas[] = {&clip, &world, &normal, &color, &rrec, &srec, &clipq, &large_list,
+                        &large_items, &wide_list, &wide_items, &large_off, &chunk_w, &keys,
+                        &shade_list, &pre, &out, &depth, &ids, &presented, &hdr, &frag_head,
+                        &touched, &frags, &olist, &olist_items, &wlist, &wlist_items, &wplots,
+                        &oscratch};
   for (DevArena *a : arenas)
     a->release();
   vertex_pool = rec_pool = clip_pool = large_pool = 0;
@@ -383,11 +384,10 @@ void LaunchCore::trim() {
 uint64_t LaunchCore::device_bytes() const {
   const DevArena *arenas[] = {&d_views, &d_frames, &d_view_draws, &d_ctr, &d_status, &d_posts,
                               &d_post_views, &d_draws, &d_scenes, &clip, &world, &normal, &color,
-                              &rrec, &srec, &clipq, &large_list, &large_items, &wide_list, &wide_items, &large_off,
-                              &chunk_w, &keys,
-                              &shade_list, &pre, &out, &depth, &ids, &presented, &hdr,
-                              &frag_head, &touched, &frags, &olist, &olist_items, &wlist,
-                              &wlist_items, &wplots, &oscratch};
+                              &rrec, &srec, &clipq, &large_list, &large_items, &wide_list,
+                              &wide_items, &large_off, &chunk_w, &keys, &shade_list, &pre, &out,
+                              &depth, &ids, &presented, &hdr, &frag_head, &touched, &frags, &olist,
+                              &olist_items, &wlist, &wlist_items, &wplots, &oscratch};
   uint64_t t = 0;
   for (const DevArena *a : arenas)
     t += a->cap;

@@ -1322,9 +1322,9 @@ __device__ __forceinline__ void fold3(float w[3], const float d[3], int k) {
  * wide one.  Every
  * chunk's edge values at its first sample are exact folds; they stay in
  * chunk_w, so that shading one of its samples folds at most 31 steps instead
- * of again from the record's corner (64 views' shading 3.83 -> 2.97 ms).  Chunks with a sample that may be
- * covered go through a queue in shared memory and are walked 32 at a time,
- * a lane each, so that empty ones (about half of a wide triangle's box) take
+ * of again from the record's corner (64 views' shading 3.83 -> 2.97 ms).
+ * Chunks with a sample that may be covered go through a queue in shared memory
+ * and are walked 32 at a time, a lane each, so that empty ones (about half of a wide triangle's box) take
  * no lane.
  * As independent (row, chunk) items of a thread each, every chunk folded
  * both ways from the corner and searched its record alone: a ground plane of
@@ -1472,7 +1472,8 @@ __device__ __forceinline__ void narrow_rows(const FrameArgs &a, uint32_t base, L
  * chunk's start: the long folds run once per row and band. */
 __device__ __forceinline__ void wide_band(const FrameArgs &a, uint32_t it, LargeSmem &q,
                                           uint32_t &n) {
-  static_assert(BAND_ROWS == 8 && BAND_CHUNKS == 8, "a lane per row and value, two chunks per lane");
+  static_assert(BAND_ROWS == 8 && BAND_CHUNKS == 8,
+                "a lane per row and value, two chunks per lane");
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t slot = warp_slot(a.wide_items, min(a.ctr->wide_count, a.large_cap), it);
   const uint32_t rid = a.wide_list[slot];
@@ -1881,10 +1882,11 @@ __device__ __forceinline__ uint32_t shade_fixed(uint32_t n, uint32_t step) {
 /* 4 blocks of 256 per SM (64 registers): the kernel is issue-bound and the
  * extra warps hide the dependent-latency stalls of the lighting chains. */
 /* With keys_next set, the kernel also clears the next frame's key buffer
- * (keys alternate between two buffers): 16-byte stores g + m * step (g the
- * thread's index, step the grid's threads), two per shaded sample and the
- * rest after the last one, so the writes spread over a kernel whose time is
- * arithmetic, and no frame waits for a clear of its own. */
+ * (keys alternate between two buffers): the warp that shades the 32 samples
+ * from `base` on stores the 64 16-byte groups from 2 * base on, two a lane, and
+ * the groups behind the last sample's are stored after the loop, so the writes
+ * spread over a kernel whose time is arithmetic, and no frame waits for a clear
+ * of its own. */
 template <bool SH>
 __global__ void __launch_bounds__(256, 4) k_shade(FrameArgs a) {
   pdl_wait();
@@ -1925,9 +1927,10 @@ __global__ void __launch_bounds__(256, 4) k_shade(FrameArgs a) {
 /* ------------------------------------------------------------------------
  * k_post — FXAA (rasterizer.c:2625-2761), tonemap/gamma/vignette
  * (postprocess.c:24-116) and the SSAA box (viewport.c:3385-3411).  A block
- * of 32x8 threads owns 32x8 presented pixels: it stages their samples plus
- * a one-sample halo (and each sample's luma) in shared memory with
- * coalesced loads, then each thread filters its ssaa x ssaa samples.
+ * of 32x8 threads owns a tile of 32x8 presented pixels (32x32 at SSAA 1): it
+ * stages their samples plus a one-sample halo (and each sample's luma) in
+ * shared memory with coalesced loads, then each thread filters its pixel's
+ * ssaa x ssaa samples (its four pixels' at SSAA 1).
  * ------------------------------------------------------------------------ */
 __device__ __forceinline__ float luma(uchar4 p) {
   return 0.299f * (float)p.x + 0.587f * (float)p.y + 0.114f * (float)p.z;
@@ -3209,9 +3212,10 @@ __device__ __noinline__ void heapsort_keys(ulonglong2 *h, uint32_t n) {
  * ORDERED_MAX_FRAGS are gathered and insertion-sorted in registers; a
  * longer list is copied with its keys into the fold's scratch and heapsorted
  * there, or in a wireframe frame left to a warp of its own (keys are
- * distinct: a record covers a sample once, a line plot is one item).  WIRE: the launch has line plots, which sort by frag_key (a
- * triangle's plots in the reference's drawing order after the triangles
- * before it); fragments then travel as (key, node), others as their order. */
+ * distinct: a record covers a sample once, a line plot is one item).  WIRE:
+ * the launch has line plots, which sort by frag_key (a triangle's plots in the
+ * reference's drawing order after the triangles before it); fragments then
+ * travel as (key, node), others as their order. */
 template <bool SH, bool WIRE>
 __device__ __forceinline__ void ofold_apply(const FrameArgs &a, OFold &st, int x, int y,
                                             unsigned long long key, uint32_t v) {

@@ -160,15 +160,13 @@ extern "C" void mopcuda_device_destroy(MopCudaDevice *d) {
     return;
   cudaSetDevice(d->ordinal);
   mc_stream_sync(d, 10000);
-  DevArena *arenas[] = {&d->irr,      &d->pf,         &d->brdf,        &d->d_draws,
-                        &d->d_lights, &d->clip,       &d->world,       &d->normal,
-                        &d->color,    &d->rrec,       &d->srec,
-                        &d->clipq,    &d->keys[0],    &d->keys[1],     &d->large_lists,
-                        &d->chunk_w,
-                        &d->shade_list, &d->counters, &d->pick_xy,     &d->pick_out,
-                        &d->deform_params, &d->hdr, &d->frag_head, &d->frags, &d->touched,
-                        &d->olist, &d->olist_items, &d->wlist, &d->wlist_items, &d->wplots, &d->oscratch, &d->sh_map[0], &d->sh_map[1], &d->sh_d_draws,
-                        &d->sh_recs, &d->sh_items, &d->sh_ctr, &d->env, &d->ibl_tab};
+  DevArena *arenas[] = {&d->irr, &d->pf, &d->brdf, &d->d_draws, &d->d_lights, &d->clip, &d->world,
+                        &d->normal, &d->color, &d->rrec, &d->srec, &d->clipq, &d->keys[0],
+                        &d->keys[1], &d->large_lists, &d->chunk_w, &d->shade_list, &d->counters,
+                        &d->pick_xy, &d->pick_out, &d->deform_params, &d->hdr, &d->frag_head,
+                        &d->frags, &d->touched, &d->olist, &d->olist_items, &d->wlist,
+                        &d->wlist_items, &d->wplots, &d->oscratch, &d->sh_map[0], &d->sh_map[1],
+                        &d->sh_d_draws, &d->sh_recs, &d->sh_items, &d->sh_ctr, &d->env, &d->ibl_tab};
   for (DevArena *a : arenas)
     a->release();
   d->h_ibl.release();

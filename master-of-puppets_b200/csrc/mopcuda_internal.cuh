@@ -181,9 +181,9 @@ static_assert(sizeof(Counters) % 8 == 0 && offsetof(Counters, large_items) % 8 =
  * longer ones are folded by a warp each. */
 #define WIRE_THREAD_FRAGS 24
 
-/* Records whose clamped bbox exceeds these bounds are rasterised as
- * (row, RASTER_CHUNK-sample) items spread over many threads; smaller ones
- * by one thread each. */
+/* Records whose clamped bbox exceeds these bounds are rasterised a warp at a
+ * time, RASTER_CHUNK samples of a row per lane; smaller ones by one thread
+ * each. */
 #define SMALL_MAX_SIDE 32  /* default small-record limits */
 #define SMALL_MAX_AREA 128
 #define RASTER_CHUNK 32
