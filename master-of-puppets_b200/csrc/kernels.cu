@@ -31,7 +31,9 @@
  * completed and its writes are visible (griddepcontrol.wait).  A kernel
  * launched without the attribute passes pdl_wait() at once, so the kernels
  * stay correct wherever they are launched from.  No kernel triggers early:
- * a successor starts once all of its predecessor's blocks have exited.
+ * a successor starts once all of its predecessor's blocks have exited.  What a
+ * kernel of the frame writes is never read with __ldg: that load is for memory
+ * no one writes while the kernel runs, and may move ahead of the wait.
  * (Triggering after the wait, so that successors' blocks take the room as it
  * comes free, made every frame 6-9 % slower.) */
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -2277,7 +2279,7 @@ __device__ __forceinline__ void post_pixel(const PostArgs &a, const uchar4 (*s_c
         c = fxaa_blend<TW>(s_c, s_l, ti0 + i, tj0 + j, c, range, lM, lN, lS, lW, lE);
     }
     if (FOG) {
-      c = post_fog_sample(a, s_thr, c, __ldg(a.depth + (size_t)y * w + x),
+      c = post_fog_sample(a, s_thr, c, a.depth[(size_t)y * w + x],
                           (a.effects & 4u) ? vignette(x, y) : 1.0f);
     } else if (a.effects != 0u && !(a.effects & 4u)) {
       /* without vignette the post-process is a fixed byte map */
@@ -2771,7 +2773,7 @@ __device__ __forceinline__ void oraster_item(const FrameArgs &a, uint32_t it, ui
         const float b0 = w0 * r.inv_area, b1 = w1 * r.inv_area, b2 = w2 * r.inv_area;
         zz = b0 * r.zc[0] + b1 * r.zc[1] + b2 * r.zc[2];
       }
-      if (a.ordered_keep_all || zz < __ldg(a.depth + row + i))
+      if (a.ordered_keep_all || zz < a.depth[row + i])
         m |= 1u << i;
     }
     w0 = __fadd_rn(w0, r.dx[0]);
